@@ -94,6 +94,7 @@ template <typename T> struct JobState {
     C *data = nullptr, *y = nullptr, *r = nullptr, *v = nullptr, *z = nullptr, *p = nullptr,
       *q = nullptr, *slices = nullptr;
     int *known = nullptr;
+    void *diff = nullptr;  // diffusion scratch
     double *part = nullptr, *dots = nullptr, *tv_part = nullptr, *tv_scal = nullptr,
            *rh = nullptr;
     int part_stride = 0, tv_cap = 0;
@@ -217,6 +218,14 @@ template <typename T> static int zfft(nudim_job *jb, JobState<T> &s, int dir)
 }
 
 // ================================================================ job state setup
+// the diffusion's parameters (reconstruction.c:627, reconstruction-parallel.c:766)
+static float job_lambda(const nudim_job_desc &d)
+{
+    return d.variant == NUDIM_VARIANT_PARALLEL ? 0.4f : 0.25f;
+}
+constexpr float kJobKappa = 0.005f;
+constexpr int kJobSweeps = 80;
+
 // The CGNR form of a job state: NFFT (a trafo and an adjoint per step, the
 // reference's own route and the FP64 default) or Toeplitz (one convolution
 // pass per step, the FP32 default where the plan's grid allows it);
@@ -286,6 +295,12 @@ template <typename T> static int state_init(nudim_job *jb, JobState<T> &s)
         s.tv_cap = tv_part_count(nz, np, np);
         NUDIM_TRY(s.alloc(&s.tv_part, s.tv_cap));
         NUDIM_TRY(s.alloc(&s.tv_scal, 4));
+    }
+    if (jb->d.denoise == NUDIM_DENOISE_DIFFUSION) {
+        const size_t db = diffusion_scratch<T>(nz, np, np, job_lambda(jb->d), kJobKappa, kJobSweeps);
+        char *q = nullptr;
+        if (db) NUDIM_TRY(s.alloc(&q, db));
+        s.diff = q;
     }
     s.part_stride = cgnr_part_stride(M, (int)P2);
     NUDIM_TRY(s.alloc(&s.part, (size_t)nz * s.part_stride + 2 * (size_t)nz + 2));
@@ -387,9 +402,9 @@ template <typename T> static int iterate_body(nudim_job *jb, JobState<T> &s, boo
         NUDIM_CUDA(cudaStreamSynchronize(st));
     }
     if (d.denoise == NUDIM_DENOISE_DIFFUSION) {
-        float lam = d.variant == NUDIM_VARIANT_PARALLEL ? 0.4f : 0.25f;
         ProfScope ps(jb->ctx, PK_DIFFUSION, st, 2.0 * sT * (double)V);
-        NUDIM_TRY(diffusion_run<T>(s.img_b, nz, np, np, nz, lam, 0.005f, 80, st));
+        NUDIM_TRY(diffusion_run<T>(s.img_b, nz, np, np, nz, job_lambda(d), kJobKappa, kJobSweeps,
+                                   s.diff, st));
     } else if (d.denoise == NUDIM_DENOISE_TV) {
         bool h = d.height && d.variant == NUDIM_VARIANT_SERIAL;
         int ylo = (2 * d.ncenter - d.nheight) / 2, yhi = (2 * d.ncenter + d.nheight) / 2;
@@ -681,6 +696,12 @@ static size_t job_bytes(const nudim_job_desc *d, int A, bool both, size_t fused_
         size_t sC = 2 * sT;
         size_t b = 3 * V * sT + 3 * V * sC + 4 * nz * M * sC;  // + the initial volume
         if (d->denoise == NUDIM_DENOISE_TV) b += V * sT;
+        if (d->denoise == NUDIM_DENOISE_DIFFUSION) {
+            const float lam = job_lambda(*d);
+            b += sT == 4 ? diffusion_scratch<float>(d->nz, d->np, d->np, lam, kJobKappa, kJobSweeps)
+                         : diffusion_scratch<double>(d->nz, d->np, d->np, lam, kJobKappa,
+                                                     kJobSweeps);
+        }
         b += M * (8 + 28 * sT + 20);  // node tables and tile lists
         // fused-path lists: ~11 adjoint tile entries and <= 5 trafo entries per
         // node (4-column blocks): id + 12 weights, and 3 ints + 20 weights
@@ -747,6 +768,7 @@ int nudim_ctx_destroy(nudim_ctx *c)
     for (auto &kv : c->fftz) cufftDestroy(kv.second);
     cudaFree(c->ws);
     cudaFree(c->scratch);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
     cudaStreamDestroy(c->stream);
     delete c;
     return NUDIM_OK;
@@ -1518,9 +1540,26 @@ int nudim_diffusion2d(nudim_ctx *ctx, int precision, void *vol, int nz, int ny, 
     }
     NUDIM_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
-    if (precision == NUDIM_FP64)
-        return diffusion_run<double>((double *)vol, nz, ny, nx, nx_bound, lambda, kappa, niter, st);
-    return diffusion_run<float>((float *)vol, nz, ny, nx, nx_bound, lambda, kappa, niter, st);
+    // scratch from the context's stream-ordered pool; without room for it the
+    // forms that need none run
+    const size_t nb = precision == NUDIM_FP64
+                          ? diffusion_scratch<double>(nz, ny, nx, lambda, kappa, niter)
+                          : diffusion_scratch<float>(nz, ny, nx, lambda, kappa, niter);
+    void *scr = nullptr;
+    if (nb) {
+        cudaMemPool_t pool;
+        NUDIM_TRY(ctx_pool(ctx, &pool));
+        if (cudaMallocFromPoolAsync(&scr, nb, pool, st) != cudaSuccess) {
+            cudaGetLastError();
+            scr = nullptr;
+        }
+    }
+    const int rc =
+        precision == NUDIM_FP64
+            ? diffusion_run<double>((double *)vol, nz, ny, nx, nx_bound, lambda, kappa, niter, scr, st)
+            : diffusion_run<float>((float *)vol, nz, ny, nx, nx_bound, lambda, kappa, niter, scr, st);
+    if (scr) cudaFreeAsync(scr, st);
+    return rc;
 }
 
 }  // extern "C"

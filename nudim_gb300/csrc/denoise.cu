@@ -475,8 +475,10 @@ __device__ __forceinline__ T diff_cell(T cv, T nN, T nS, T nE, T nW, T lambda, T
 // This form works in global memory (any plane size).
 template <typename T>
 __global__ void __launch_bounds__(1024)
-k_diffusion(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, int niter)
+k_diffusion(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, int niter,
+            const int *__restrict__ only)
 {
+    if (only && !only[blockIdx.x]) return;
     T *U = u + (size_t)blockIdx.x * ny * nx;
     const T lambda = (T)lambda_d, Ksq = (T)ksq_d;
     int D = ny + nx - 1, L = min(ny, nx);
@@ -522,8 +524,9 @@ constexpr int kDiffMaxG = 64;  // sweeps per group (task tables in shared memory
 template <typename T>
 __global__ void __launch_bounds__(1024)
 k_diffusion_ring(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, int niter,
-                 int G, int R)
+                 int G, int R, const int *__restrict__ only)
 {
+    if (only && !only[blockIdx.x]) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T *ring = (T *)smraw;
     T *U = u + (size_t)blockIdx.x * ny * nx;
@@ -817,8 +820,9 @@ k_diffusion_rows(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, i
 template <typename T, int TPR>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 768 : 1024, sizeof(T) == 4 ? 2 : 1)
 k_diffusion_pairs(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, int niter,
-                  int G, int R, int S)
+                  int G, int R, int S, const int *__restrict__ only)
 {
+    if (only && !only[blockIdx.x]) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T *ring = (T *)smraw;  // R slots of S >= ny + 1 values (S even)
     T *U = u + (size_t)blockIdx.x * ny * nx;
@@ -952,29 +956,47 @@ k_diffusion_pairs(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, 
 // NUDIM_DIFFUSION=pairs|rows|tables selects one.  All give the same cells bit
 // for bit.  Read at every launch (a captured graph keeps the form it was
 // captured with).
-enum DiffForm { DF_PAIRS, DF_ROWS, DF_TABLES };
+enum DiffForm { DF_STRIPS, DF_PAIRS, DF_ROWS, DF_TABLES };
 template <typename T> static DiffForm diffusion_form()
 {
     const char *e = getenv("NUDIM_DIFFUSION");
+    if (e && !strcmp(e, "strips") && sizeof(T) == 4) return DF_STRIPS;
     if (e && !strcmp(e, "tables")) return DF_TABLES;
     if (e && !strcmp(e, "rows")) return DF_ROWS;
     if (e && !strcmp(e, "pairs")) return DF_PAIRS;
-    return sizeof(T) == 8 ? DF_TABLES : DF_PAIRS;
+    return sizeof(T) == 8 ? DF_TABLES : DF_STRIPS;
+}
+
+template <typename T>
+size_t diffusion_scratch(int nz, int ny, int nx, float lambda, float kappa, int niter)
+{
+    if (sizeof(T) == 8 || nz <= 0 || diffusion_form<T>() != DF_STRIPS ||
+        !strips_fits(ny, nx, niter, lambda, (double)kappa * (double)kappa))
+        return 0;
+    return strips_scratch(nz, ny, nx, niter);
 }
 
 template <typename T>
 int diffusion_run(T *u, int nz, int ny, int nx, int nx_bound, float lambda, float kappa,
-                  int niter, cudaStream_t st)
+                  int niter, void *scratch, cudaStream_t st)
 {
     if (niter <= 0 || nz <= 0) return NUDIM_OK;
     double ksq = (double)kappa * (double)kappa;
+    DiffForm form = diffusion_form<T>();
+    const int *only = nullptr;  // pairs form: the planes the strips left to it
+    if constexpr (sizeof(T) == 4) {
+        if (form == DF_STRIPS && scratch && strips_fits(ny, nx, niter, lambda, ksq)) {
+            NUDIM_TRY(strips_run(u, nz, ny, nx, nx_bound, lambda, ksq, niter, scratch, st));
+            only = (const int *)scratch;
+        }
+    }
+    if (form == DF_STRIPS) form = DF_PAIRS;
     int L = ny < nx ? ny : nx;
     int P = std::min(1024, (L + 31) & ~31);
     // FP32 on planes up to 512 wide: two CTAs per SM; otherwise one CTA with
     // up to 160 KB of ring
     bool two = sizeof(T) == 4 && P <= 512;
     const size_t budget = two ? ((size_t)108 << 10) : ((size_t)160 << 10);
-    const DiffForm form = diffusion_form<T>();
     const int cap = sizeof(T) == 4 ? 768 : 1024;
     if (form == DF_PAIRS) {
         // two rows per thread: slots of S = ny + 1 rounded up to even values;
@@ -995,7 +1017,7 @@ int diffusion_run(T *u, int nz, int ny, int nx, int nx_bound, float lambda, floa
         NUDIM_CUDA(cudaFuncSetAttribute(k_diffusion_pairs<T, TP>,                               \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 160 << 10)); \
         k_diffusion_pairs<T, TP><<<nz, threads, smem, st>>>(u, ny, nx, nx_bound, (double)lambda, \
-                                                             ksq, niter, G, R, S);              \
+                                                             ksq, niter, G, R, S, only);        \
     } while (0)
             if (tpr == 8) NUDIM_DIFF_PAIRS(8);
             else if (tpr == 4) NUDIM_DIFF_PAIRS(4);
@@ -1046,9 +1068,10 @@ int diffusion_run(T *u, int nz, int ny, int nx, int nx_bound, float lambda, floa
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         160 << 10));
         k_diffusion_ring<T><<<nz, threads, smem, st>>>(u, ny, nx, nx_bound, (double)lambda, ksq,
-                                                        niter, G, R);
+                                                        niter, G, R, only);
     } else {
-        k_diffusion<T><<<nz, 1024, 0, st>>>(u, ny, nx, nx_bound, (double)lambda, ksq, niter);
+        k_diffusion<T><<<nz, 1024, 0, st>>>(u, ny, nx, nx_bound, (double)lambda, ksq, niter,
+                                     only);
     }
     NUDIM_LAUNCH_CHECK();
     return NUDIM_OK;
@@ -1058,7 +1081,11 @@ template int tv_run<double>(double *, double *, double *, int, double *, int, in
                             int, int, int, int, cudaStream_t, double *, double *);
 template int tv_run<float>(float *, float *, double *, int, double *, int, int, int, float, int,
                            int, int, int, cudaStream_t, float *, float *);
-template int diffusion_run<double>(double *, int, int, int, int, float, float, int, cudaStream_t);
-template int diffusion_run<float>(float *, int, int, int, int, float, float, int, cudaStream_t);
+template int diffusion_run<double>(double *, int, int, int, int, float, float, int, void *,
+                                   cudaStream_t);
+template int diffusion_run<float>(float *, int, int, int, int, float, float, int, void *,
+                                  cudaStream_t);
+template size_t diffusion_scratch<double>(int, int, int, float, float, int);
+template size_t diffusion_scratch<float>(int, int, int, float, float, int);
 
 }  // namespace nudim

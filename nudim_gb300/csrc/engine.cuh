@@ -62,6 +62,10 @@ struct nudim_ctx {
     std::map<std::tuple<int, int, int, int>, std::pair<int, int>> tuned;
     std::map<std::tuple<int, int, int, int>, cufftHandle> fft2d;  // n0,n1,batch,prec
     std::map<std::tuple<int, int, int, int>, cufftHandle> fftz;   // nz,P2,prec,kind
+    // stream-ordered scratch of the operator-level diffusion: each call takes
+    // its own from here and gives it back, so calls on several streams share
+    // nothing; up to kPoolKeep bytes stay with the pool between calls
+    cudaMemPool_t pool = nullptr;
     double *scratch = nullptr;   // small reduction workspace (operator-level calls)
     size_t scratch_bytes = 0;
 };
@@ -98,6 +102,8 @@ int prof_collect(nudim_ctx *c);
 int ctx_workspace(nudim_ctx *ctx, size_t bytes, void **p);
 int upload_async(void **dst, const void *src, size_t nb, cudaStream_t st);
 int ctx_scratch(nudim_ctx *ctx, size_t bytes, double **p);
+int ctx_pool(nudim_ctx *ctx, cudaMemPool_t *pool);
+constexpr unsigned long long kPoolKeep = 512ull << 20;
 int ctx_fft2d(nudim_ctx *ctx, int n0, int n1, int batch, int prec, cufftHandle *h);
 
 template <typename T> cufftType fft_c2c();
@@ -300,8 +306,21 @@ int tv_part_count(int nz, int ny, int nx);
 // them) -> S [nz][ns*np] (device); scratch of the X contraction <= budget.
 int dft_slices(const double *dens, int nx, int ny, int nz, int np, const double *x2, int ns,
                double2 *S, size_t budget, cudaStream_t st);
+// scratch: diffusion_scratch() bytes for the same shape, or nullptr (the forms
+// that need none run then); not shared with work that may overlap
 template <typename T>
 int diffusion_run(T *u, int nz, int ny, int nx, int nx_bound, float lambda, float kappa,
-                  int niter, cudaStream_t st);
+                  int niter, void *scratch, cudaStream_t st);
+template <typename T>
+size_t diffusion_scratch(int nz, int ny, int nx, float lambda, float kappa, int niter);
+
+// strips.cu: the diffusion with its wavefront in registers.  flags (the
+// scratch's head): planes it leaves untouched because a value is beyond its
+// range
+bool strips_fits(int ny, int nx, int niter, double lambda, double ksq);
+size_t strips_scratch(int nz, int ny, int nx, int niter);
+inline size_t strips_flag_bytes(int nz) { return ((size_t)nz * sizeof(int) + 255) & ~(size_t)255; }
+int strips_run(float *u, int nz, int ny, int nx, int nxb, double lambda, double ksq, int niter,
+               void *scratch, cudaStream_t st);
 
 }  // namespace nudim

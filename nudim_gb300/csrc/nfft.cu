@@ -122,6 +122,21 @@ int ctx_scratch(nudim_ctx *ctx, size_t bytes, double **p)
     return NUDIM_OK;
 }
 
+int ctx_pool(nudim_ctx *ctx, cudaMemPool_t *pool)
+{
+    if (!ctx->pool) {
+        cudaMemPoolProps pr = {};
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = ctx->device;
+        unsigned long long keep = kPoolKeep;
+        NUDIM_CUDA(cudaMemPoolCreate(&ctx->pool, &pr));
+        NUDIM_CUDA(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    *pool = ctx->pool;
+    return NUDIM_OK;
+}
+
 int ctx_fft2d(nudim_ctx *ctx, int n0, int n1, int batch, int prec, cufftHandle *h)
 {
     auto key = std::make_tuple(n0, n1, batch, prec);
