@@ -950,30 +950,31 @@ k_diffusion_pairs(T *u, int ny, int nx, int nxb, double lambda_d, double ksq_d, 
     }
 }
 
-// The wavefront form: pairs (k_diffusion_pairs, the FP32 default), rows
-// (k_diffusion_rows) or task tables (k_diffusion_ring, the FP64 default: the
-// FP64 pipe bounds every form there and the tables form measured fastest);
-// NUDIM_DIFFUSION=pairs|rows|tables selects one.  All give the same cells bit
-// for bit.  Read at every launch (a captured graph keeps the form it was
-// captured with).
+// The wavefront form: strips (strips.cu, the default where its range and the
+// scratch allow), pairs (k_diffusion_pairs, FP32 otherwise), rows
+// (k_diffusion_rows) or task tables (k_diffusion_ring, FP64 otherwise);
+// NUDIM_DIFFUSION=strips|pairs|rows|tables selects one.  FP64: all give the
+// same cells bit for bit; FP32: the last three, while the strips pair their
+// coefficients' denominators.  Read at every launch (a captured graph keeps the
+// form it was captured with).
 enum DiffForm { DF_STRIPS, DF_PAIRS, DF_ROWS, DF_TABLES };
 template <typename T> static DiffForm diffusion_form()
 {
     const char *e = getenv("NUDIM_DIFFUSION");
-    if (e && !strcmp(e, "strips") && sizeof(T) == 4) return DF_STRIPS;
+    if (e && !strcmp(e, "strips")) return DF_STRIPS;
     if (e && !strcmp(e, "tables")) return DF_TABLES;
     if (e && !strcmp(e, "rows")) return DF_ROWS;
     if (e && !strcmp(e, "pairs")) return DF_PAIRS;
-    return sizeof(T) == 8 ? DF_TABLES : DF_STRIPS;
+    return DF_STRIPS;
 }
 
 template <typename T>
 size_t diffusion_scratch(int nz, int ny, int nx, float lambda, float kappa, int niter)
 {
-    if (sizeof(T) == 8 || nz <= 0 || diffusion_form<T>() != DF_STRIPS ||
-        !strips_fits(ny, nx, niter, lambda, (double)kappa * (double)kappa))
+    if (nz <= 0 || diffusion_form<T>() != DF_STRIPS ||
+        !strips_fits<T>(ny, nx, niter, lambda, (double)kappa * (double)kappa))
         return 0;
-    return strips_scratch(nz, ny, nx, niter);
+    return strips_scratch<T>(nz, ny, nx, niter);
 }
 
 template <typename T>
@@ -984,13 +985,12 @@ int diffusion_run(T *u, int nz, int ny, int nx, int nx_bound, float lambda, floa
     double ksq = (double)kappa * (double)kappa;
     DiffForm form = diffusion_form<T>();
     const int *only = nullptr;  // pairs form: the planes the strips left to it
-    if constexpr (sizeof(T) == 4) {
-        if (form == DF_STRIPS && scratch && strips_fits(ny, nx, niter, lambda, ksq)) {
-            NUDIM_TRY(strips_run(u, nz, ny, nx, nx_bound, lambda, ksq, niter, scratch, st));
-            only = (const int *)scratch;
-        }
+    if (form == DF_STRIPS && scratch && strips_fits<T>(ny, nx, niter, lambda, ksq)) {
+        NUDIM_TRY(strips_run<T>(u, nz, ny, nx, nx_bound, lambda, ksq, niter, scratch, st));
+        if (sizeof(T) == 8) return NUDIM_OK;
+        only = (const int *)scratch;
     }
-    if (form == DF_STRIPS) form = DF_PAIRS;
+    if (form == DF_STRIPS) form = sizeof(T) == 8 ? DF_TABLES : DF_PAIRS;
     int L = ny < nx ? ny : nx;
     int P = std::min(1024, (L + 31) & ~31);
     // FP32 on planes up to 512 wide: two CTAs per SM; otherwise one CTA with

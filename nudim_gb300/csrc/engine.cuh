@@ -317,10 +317,12 @@ size_t diffusion_scratch(int nz, int ny, int nx, float lambda, float kappa, int 
 // strips.cu: the diffusion with its wavefront in registers.  flags (the
 // scratch's head): planes it leaves untouched because a value is beyond its
 // range
+template <typename T>
 bool strips_fits(int ny, int nx, int niter, double lambda, double ksq);
-size_t strips_scratch(int nz, int ny, int nx, int niter);
+template <typename T> size_t strips_scratch(int nz, int ny, int nx, int niter);
 inline size_t strips_flag_bytes(int nz) { return ((size_t)nz * sizeof(int) + 255) & ~(size_t)255; }
-int strips_run(float *u, int nz, int ny, int nx, int nxb, double lambda, double ksq, int niter,
+template <typename T>
+int strips_run(T *u, int nz, int ny, int nx, int nxb, double lambda, double ksq, int niter,
                void *scratch, cudaStream_t st);
 
 }  // namespace nudim

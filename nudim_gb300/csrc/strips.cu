@@ -30,7 +30,8 @@
 // The cell's four coefficients K^2 / (K^2 + g^2) are summed in pairs over a
 // common denominator, gN/dN + gS/dS = (gN dS + gS dN) / (dN dS): one reciprocal
 // for two coefficients (four per cell bound the loop by the special-function
-// unit at 4 cells per clock and SM).
+// unit at 4 cells per clock and SM).  FP64 by the integer units (66 % of their
+// rate) and the FP64 unit (67 %), see intdiv.cuh.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -38,6 +39,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "intdiv.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -67,15 +69,24 @@ __device__ __forceinline__ unsigned bit_at(int s)
 constexpr float kMaxF = 1e9f;
 constexpr double kMinKsq = 1e-17, kMaxKsq = 1e18;
 
-// Cells of two adjacent rows; lk = lambda K^2.  The differences are scalar:
+template <typename T> struct CellArgs;
+template <> struct CellArgs<float> {
+    float lk, ksq;  // lambda K^2, K^2
+};
+template <> struct CellArgs<double> {
+    double lambda;
+    DiffDiv div;
+};
+
+// Cells of two adjacent rows.  The differences are scalar:
 // the rows' N and S are not a register pair, and pairing rows (i, i + R/2),
 // whose N and S are, took more moves than it saved (256 x 384 x 384: 4.15 ->
 // 4.47 ms).
 __device__ __forceinline__ void cell2(float c0, float c1, float n0, float n1, float s0, float s1,
-                                      float e0, float e1, float w0, float w1, float lk, float ksq,
-                                      float &u0, float &u1)
+                                      float e0, float e1, float w0, float w1,
+                                      const CellArgs<float> &k, float &u0, float &u1)
 {
-    const float2 k2 = make_float2(ksq, ksq);
+    const float2 k2 = make_float2(k.ksq, k.ksq);
     const float2 gN = make_float2(n0 - c0, n1 - c1), gS = make_float2(s0 - c0, s1 - c1);
     const float2 gE = make_float2(e0 - c0, e1 - c1), gW = make_float2(w0 - c0, w1 - c1);
     const float2 dN = __ffma2_rn(gN, gN, k2), dS = __ffma2_rn(gS, gS, k2);
@@ -85,9 +96,42 @@ __device__ __forceinline__ void cell2(float c0, float c1, float n0, float n1, fl
     const float2 rp = make_float2(rcp_approx(p.x), rcp_approx(p.y));
     const float2 rq = make_float2(rcp_approx(q.x), rcp_approx(q.y));
     const float2 sum = __ffma2_rn(b, rq, __fmul2_rn(a, rp));
-    const float2 u = __ffma2_rn(make_float2(lk, lk), sum, make_float2(c0, c1));
+    const float2 u = __ffma2_rn(make_float2(k.lk, k.lk), sum, make_float2(c0, c1));
     u0 = u.x;
     u1 = u.y;
+}
+
+// FP64: the reference's operations in its order, each rounded as IEEE rounds
+// it; the fluxes in integer arithmetic (intdiv.cuh), with the FP64 unit's
+// divisions for the values that does not take.
+__device__ __noinline__ double flux_divided(double g, double ksq)
+{
+    return rn_mul(rn_div(1.0, rn_add(1.0, rn_div(rn_mul(g, g), ksq))), g);
+}
+
+__device__ __forceinline__ double cell1(double c, double n, double s, double e, double w,
+                                        const CellArgs<double> &k)
+{
+    const double g[4] = {rn_sub(n, c), rn_sub(s, c), rn_sub(e, c), rn_sub(w, c)};
+    double f[4];
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < 4; j++) ok &= diff_flux_int(g[j], k.div, f + j);
+    if (!ok) {
+        f[0] = flux_divided(g[0], k.div.b);
+        f[1] = flux_divided(g[1], k.div.b);
+        f[2] = flux_divided(g[2], k.div.b);
+        f[3] = flux_divided(g[3], k.div.b);
+    }
+    return rn_add(c, rn_mul(k.lambda, rn_add(rn_add(rn_add(f[0], f[1]), f[2]), f[3])));
+}
+
+__device__ __forceinline__ void cell2(double c0, double c1, double n0, double n1, double s0,
+                                      double s1, double e0, double e1, double w0, double w1,
+                                      const CellArgs<double> &k, double &u0, double &u1)
+{
+    u0 = cell1(c0, n0, s0, e0, w0, k);
+    u1 = cell1(c1, n1, s1, e1, w1, k);
 }
 
 template <typename T, int V> struct alignas(sizeof(T) * V) Vec {
@@ -112,19 +156,20 @@ template <typename T, int V> __device__ __forceinline__ Vec<T, V> ldcg_vec(const
     return r;
 }
 
-struct StripArgs {
+template <typename T> struct StripArgs {
     int nz, ny, nx, nxb;
     int rounds, W, B, P;  // warps per band and CTA, bands of 32 R rows, slots of the scratch
     int check;            // mark the planes out of range (a call's first launch)
-    float lk, ksq;
+    CellArgs<T> cell;
 };
 
 template <typename T, int R, int Q, bool FULL, bool CL>
 __global__ void __launch_bounds__(512, 1)
 k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__ flags,
-                   StripArgs a)
+                   StripArgs<T> a)
 {
     constexpr int V = vec_of<T, R>(), NV = R / V;
+    constexpr bool FLOAT = sizeof(T) == 4;
     using Vt = Vec<T, V>;
     extern __shared__ __align__(16) unsigned char smraw[];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -177,7 +222,7 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
                 for (int j = 0; j < 32; j++) {
                     T v = T(0);
                     if (r0 + j < a.ny && x < a.nx) v = U[(size_t)(r0 + j) * a.nx + x];
-                    if (!(fabs(v) < T(kMaxF))) big = true;
+                    if (FLOAT && !(fabs(v) < T(kMaxF))) big = true;
                     tile[j * 33 + lane] = v;
                     x = x ? x - 1 : P - 1;
                 }
@@ -187,11 +232,12 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
                     if (g0 + j < P) S[(size_t)(g0 + j) * NR + r0 + lane] = tile[lane * 33 + j];
                 __syncwarp();
             }
-            if (__any_sync(0xffffffffu, big) && lane == 0 && a.check) atomicOr(flags + pl, 1);
+            if (FLOAT && a.check && __any_sync(0xffffffffu, big) && lane == 0)
+                atomicOr(flags + pl, 1);
             __threadfence();
             sync();
         }
-        if (__ldcg(flags + pl)) {  // not this form's plane: left untouched
+        if (FLOAT && __ldcg(flags + pl)) {  // not this form's plane: left untouched
             sync();
             continue;
         }
@@ -222,21 +268,30 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
         int cnt = (-1 - 2 * sw - y0) % P;
         if (cnt < 0) cnt += P;
         int d_out = -1 - 2 * (K - 1);  // diagonal the pipeline's last sweep is at
+        int d_in = -1 - 2 * sw;           // ... this warp's first sweep
         int slot_out = d_out % P;
         if (slot_out < 0) slot_out += P;
 
-        auto step = [&](auto phc) {
+        // One step, the exchange buffer `par` in and the other out.  ph: which of
+        // X's two is the newest; the FP32 loop alternates it, the FP64 loop
+        // (whose step is long) moves the values and keeps one copy of the code.
+        auto step = [&](auto phc, int par) {
             constexpr int ph = decltype(phc)::value, pp = ph ^ 1;
-            const int bi = ph ? exbuf : 0, bo = ph ? 0 : exbuf;
+            const int bi = par ? exbuf : 0, bo = par ? 0 : exbuf;
+            // the warp has cells on its diagonals, or will in the next step
+            const bool busy = d_in + 1 >= 32 * R * b && d_in - 2 * (Q - 1) - 32 * R * (b + 1) < span;
             // this step's input becomes the newest (over the oldest)
             T inS = T(0);
+            if (!FLOAT)
+#pragma unroll
+                for (int i = 0; i < R; i++) X[0][pp][i] = X[0][ph][i];
             if (first) {
 #pragma unroll
                 for (int i = 0; i < R; i++) X[0][ph][i] = pf[i];
                 inS = pfS;
                 fetch(slot_in);
                 slot_in = slot_in + 1 == P ? 0 : slot_in + 1;
-            } else {
+            } else if (busy) {
 #pragma unroll
                 for (int k = 0; k < NV; k++) {
                     const Vt v = in[bi + k * 32];
@@ -246,6 +301,7 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
                 if (a.B > 1 && lane == 31 && b + 1 < a.B)
                     inS = ex[bi + (size_t)((b + 1) * a.W + w) * NV * 32].v[0];
             }
+            if (busy)
 #pragma unroll
             for (int q = Q - 1; q >= 0; q--) {
                 // E: newest of the stage before, C: the one before it.  For
@@ -260,7 +316,7 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
                 T nTop = __shfl_up_sync(0xffffffffu, O[R - 1], 1);
                 T sBot = __shfl_down_sync(0xffffffffu, E[0], 1);
                 if (a.B > 1) {
-                    const int eb = ph ? NW * Q : 0;
+                    const int eb = par ? NW * Q : 0;
                     if (lane == 0 && b > 0) nTop = eN[eb + ((b - 1) * a.W + w) * Q + q];
                     if (lane == 31 && b + 1 < a.B)
                         sBot = q == 0 ? inS : eS[eb + ((b + 1) * a.W + w) * Q + q];
@@ -285,17 +341,18 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
                     if (!FULL && (mS & (1u << i))) s0 = c0;
                     if ((!FULL || i + 2 == R) && (mS & (2u << i))) s1 = c1;
                     T u0, u1;
-                    cell2(c0, c1, n0, n1, s0, s1, e0, e1, w0, w1, a.lk, a.ksq, u0, u1);
+                    cell2(c0, c1, n0, n1, s0, s1, e0, e1, w0, w1, a.cell, u0, u1);
                     D[i] = u0;
                     D[i + 1] = u1;
                 }
                 if (a.B > 1) {
-                    const int eb = ph ? 0 : NW * Q;
+                    const int eb = par ? 0 : NW * Q;
                     if (lane == 31) eN[eb + (b * a.W + w) * Q + q] = D[R - 1];
                     if (lane == 0 && q + 1 < Q) eS[eb + (b * a.W + w) * Q + q + 1] = D[0];
                 }
             }
-            if (!last) {
+            if (!busy) {
+            } else if (!last) {
 #pragma unroll
                 for (int k = 0; k < NV; k++) {
                     Vt v;
@@ -323,12 +380,17 @@ k_diffusion_strips(T *__restrict__ u, T *__restrict__ scratch, int *__restrict__
             }
             cnt = cnt + 1 == P ? 0 : cnt + 1;
             d_out++;
+            d_in++;
             slot_out = slot_out + 1 == P ? 0 : slot_out + 1;
             sync();
         };
-        for (int n = 0; n < nsteps; n += 2) {
-            step(std::integral_constant<int, 0>());
-            step(std::integral_constant<int, 1>());
+        if constexpr (FLOAT) {
+            for (int n = 0; n < nsteps; n += 2) {
+                step(std::integral_constant<int, 0>(), 0);
+                step(std::integral_constant<int, 1>(), 1);
+            }
+        } else {
+            for (int n = 0; n < nsteps; n++) step(std::integral_constant<int, 0>(), n & 1);
         }
         // ---- and out of S again
         {
@@ -365,7 +427,7 @@ template <typename T, int R, int Q> size_t strips_smem(int W, int B)
 }
 
 template <typename T, int R, int Q>
-int launch_strips(T *u, T *scratch, int *flags, const StripArgs &a, int C, int clusters,
+int launch_strips(T *u, T *scratch, int *flags, const StripArgs<T> &a, int C, int clusters,
                   cudaStream_t st)
 {
     const size_t smem = strips_smem<T, R, Q>(a.W, a.B);
@@ -400,9 +462,9 @@ int launch_strips(T *u, T *scratch, int *flags, const StripArgs &a, int C, int c
     return NUDIM_OK;
 }
 
-// How a launch cuts its planes: strips of R rows (even), B bands of 32 R rows
-// (one up to 384 rows), W warps per band and CTA of Q sweeps each, C CTAs of a
-// cluster per plane: k = Q W C live sweeps.
+// How a launch cuts its planes: strips of R rows (even), B bands of 32 R rows, W
+// warps per band and CTA of Q sweeps each, C CTAs of a cluster per plane: k =
+// Q W C live sweeps.
 struct StripShape {
     int R, B, W, Q, C, k, P, clusters;
 };
@@ -416,24 +478,50 @@ int sm_count()
     return sms;
 }
 
-// The next launch's shape with `left` sweeps to go.  16 live sweeps (or what 16
-// warps hold): more of them waste more on the pipeline's ends, fewer leave the
-// SM idle (256 x 384 x 384: 8 sweeps 4.29, 10 5.09, 16 4.15, 20 5.51 ms).  Two
-// sweeps a warp halve the exchange and let two CTAs share an SM; with a plane
-// per SM or fewer, one sweep a warp on twice the warps (64 x 128 x 128: 386 ->
-// 363 us; 256 planes of 384 x 384: 4.15 -> 4.93 ms the other way round).
-// Where four CTAs a plane still find an SM each and the strips are at least 6
-// rows, a cluster of four with 40 live sweeps (33 x 151 x 203: 753 -> 586 us;
-// 16 x 64 x 64, strips of 2 rows: 154 -> 206 us, the cluster's barrier at each
-// step costs more than the rest of the step).
-StripShape strip_shape(int nz, int ny, int nx, int left)
+// rows of a band: strips of up to 12 (FP32) or 2 (FP64) rows
+template <typename T> constexpr int kBandRows = sizeof(T) == 4 ? 384 : 64;
+
+// The next launch's shape with `left` sweeps to go.
+//
+// FP32: 16 live sweeps (or what 16 warps hold): more of them waste more on the
+// pipeline's ends, fewer leave the SM idle (256 x 384 x 384: 8 sweeps 4.29, 10
+// 5.09, 16 4.15, 20 5.51 ms).  Two sweeps a warp halve the exchange and let two
+// CTAs share an SM; with a plane per SM or fewer, one sweep a warp on twice the
+// warps (64 x 128 x 128: 386 -> 363 us; 256 planes of 384 x 384: 4.15 -> 4.93
+// ms the other way round).  Where four CTAs a plane still find an SM each and
+// the strips are at least 6 rows, a cluster of four with 40 live sweeps (33 x
+// 151 x 203: 753 -> 586 us; 16 x 64 x 64, strips of 2 rows: 154 -> 206 us, the
+// cluster's barrier at each step costs more than the rest of the step).
+//
+// FP64: the step is long (integer and FP64 units; 64 x 128 x 128: 38.0 ms for
+// the tables form with the FP64 unit's divisions, 4.0 here) and a plane on one
+// SM leaves the others idle, so a plane takes a cluster of as many CTAs as
+// bring the turns per SM down (64 planes: 1 CTA 7.3 ms, 2 4.05, 4 3.96, 8 3.98;
+// 32: 4 2.64, 8 2.54; equal turns: the smaller one), strips of 2 rows on up to
+// 16 warps (strips of 4 on half the warps: 6.6 against 5.3 ms, one warp's
+// dependent instructions bound it), 16 live sweeps; 40 where there are fewer
+// planes than clusters of 8 (9 x 100 x 130: 1.93 -> 1.71 ms).
+template <typename T> StripShape strip_shape(int nz, int ny, int nx, int left)
 {
     StripShape s;
-    s.B = (ny + 383) / 384;
+    s.B = (ny + kBandRows<T> - 1) / kBandRows<T>;
     const int r = (ny + 32 * s.B - 1) / (32 * s.B), sms = sm_count();
     s.R = r + (r & 1);
     s.C = 1;
-    if (s.B == 1 && s.R >= 6 && 4 * nz <= sms && left >= 40) {
+    if (sizeof(T) == 8) {
+        s.Q = 1;
+        auto turns = [&](int c) { return (nz * c + sms - 1) / sms; };
+        for (int c = 2; c <= 8 && 2 * c <= left; c *= 2)
+            if (turns(c) * s.C < turns(s.C) * c) s.C = c;
+        const int most = s.C == 8 && turns(8) == 1 && left >= 40 ? 40 : 16;
+        s.W = std::max(1, std::min({16 / s.B, most / s.C, left / s.C}));
+        for (int w = s.W; 2 * w > s.W; w--)
+            if (left % (w * s.C) == 0) {
+                s.W = w;
+                break;
+            }
+        s.k = s.W * s.C;
+    } else if (s.B == 1 && s.R >= 6 && 4 * nz <= sms && left >= 40) {
         s.C = 4;
         s.k = 40;
         s.Q = 1;
@@ -451,38 +539,73 @@ StripShape strip_shape(int nz, int ny, int nx, int left)
     return s;
 }
 
+bool cell_args(double lambda, double ksq, CellArgs<float> *c)
+{
+    c->ksq = (float)ksq;
+    c->lk = (float)lambda * (float)ksq;
+    return true;
+}
+bool cell_args(double lambda, double ksq, CellArgs<double> *c)
+{
+    c->lambda = lambda;
+    return diff_div_init(ksq, &c->div);
+}
+
+// strips of RR rows, if the form has them in this precision
+template <typename T, int RR>
+int launch_rows(const StripShape &s, T *u, T *S, int *flags, const StripArgs<T> &a, cudaStream_t st)
+{
+    if constexpr (sizeof(T) == 8) {
+        if constexpr (RR <= 2) return launch_strips<T, RR, 1>(u, S, flags, a, s.C, s.clusters, st);
+        set_error("diffusion: no strip of %d rows", RR);
+        return NUDIM_EINVAL;
+    } else {
+        return s.Q == 2 ? launch_strips<T, RR, 2>(u, S, flags, a, s.C, s.clusters, st)
+                        : launch_strips<T, RR, 1>(u, S, flags, a, s.C, s.clusters, st);
+    }
+}
+
 }  // namespace
 
-// The form's range: |lambda| small enough that the sweeps keep values within
-// the pair form's bounds (a sweep moves a value by at most 2 |lambda| K).
+// The form's range.  FP32: |lambda| small enough that the sweeps keep values
+// within the pair form's bounds (a sweep moves a value by at most 2 |lambda| K).
+template <typename T>
 bool strips_fits(int ny, int nx, int niter, double lambda, double ksq)
 {
-    return ny >= 1 && nx >= 1 && ny <= 384 * 16 && niter >= 1 && ksq >= kMinKsq &&
-           ksq <= kMaxKsq && std::fabs(lambda) * std::sqrt(ksq) * 2 * niter < 0.1 * kMaxF;
+    if (ny < 1 || nx < 1 || ny > kBandRows<T> * 16 || niter < 1) return false;
+    CellArgs<T> c;
+    if (sizeof(T) == 8) return cell_args(lambda, ksq, &c);
+    return ksq >= kMinKsq && ksq <= kMaxKsq &&
+           std::fabs(lambda) * std::sqrt(ksq) * 2 * niter < 0.1 * kMaxF;
 }
 
 // scratch of strips_run: a flag per plane, then a skewed plane per cluster
-size_t strips_scratch(int nz, int ny, int nx, int niter)
+template <typename T> size_t strips_scratch(int nz, int ny, int nx, int niter)
 {
     size_t most = 0;
     for (int left = niter; left > 0;) {
-        const StripShape s = strip_shape(nz, ny, nx, left);
-        most = std::max(most, sizeof(float) * (size_t)s.clusters * s.P * 32 * s.R * s.B);
+        const StripShape s = strip_shape<T>(nz, ny, nx, left);
+        most = std::max(most, sizeof(T) * (size_t)s.clusters * s.P * 32 * s.R * s.B);
         left -= left / s.k * s.k;
     }
     return most + strips_flag_bytes(nz);
 }
 
-int strips_run(float *u, int nz, int ny, int nx, int nxb, double lambda, double ksq, int niter,
+template <typename T>
+int strips_run(T *u, int nz, int ny, int nx, int nxb, double lambda, double ksq, int niter,
                void *scratch, cudaStream_t st)
 {
     int *flags = (int *)scratch;
-    float *S = (float *)((char *)scratch + strips_flag_bytes(nz));
-    NUDIM_CUDA(cudaMemsetAsync(flags, 0, strips_flag_bytes(nz), st));
+    T *S = (T *)((char *)scratch + strips_flag_bytes(nz));
+    StripArgs<T> a;
+    if (!cell_args(lambda, ksq, &a.cell)) {
+        set_error("diffusion: kappa out of the strip form's range");
+        return NUDIM_EINVAL;
+    }
+    if (sizeof(T) == 4) NUDIM_CUDA(cudaMemsetAsync(flags, 0, strips_flag_bytes(nz), st));
     for (int left = niter; left > 0;) {
-        const StripShape s = strip_shape(nz, ny, nx, left);
+        const StripShape s = strip_shape<T>(nz, ny, nx, left);
         const int rounds = left / s.k;
-        StripArgs a;
         a.nz = nz;
         a.ny = ny;
         a.nx = nx;
@@ -492,28 +615,29 @@ int strips_run(float *u, int nz, int ny, int nx, int nxb, double lambda, double 
         a.B = s.B;
         a.P = s.P;
         a.check = left == niter;
-        a.ksq = (float)ksq;
-        a.lk = (float)lambda * (float)ksq;
         int rc = NUDIM_EINVAL;
-#define NUDIM_STRIP_R(RR)                                                                        \
-    case RR:                                                                                     \
-        rc = s.Q == 2 ? launch_strips<float, RR, 2>(u, S, flags, a, s.C, s.clusters, st)         \
-                      : launch_strips<float, RR, 1>(u, S, flags, a, s.C, s.clusters, st);        \
-        break
         switch (s.R) {
-            NUDIM_STRIP_R(2);
-            NUDIM_STRIP_R(4);
-            NUDIM_STRIP_R(6);
-            NUDIM_STRIP_R(8);
-            NUDIM_STRIP_R(10);
-            NUDIM_STRIP_R(12);
+        case 2: rc = launch_rows<T, 2>(s, u, S, flags, a, st); break;
+        case 4: rc = launch_rows<T, 4>(s, u, S, flags, a, st); break;
+        case 6: rc = launch_rows<T, 6>(s, u, S, flags, a, st); break;
+        case 8: rc = launch_rows<T, 8>(s, u, S, flags, a, st); break;
+        case 10: rc = launch_rows<T, 10>(s, u, S, flags, a, st); break;
+        case 12: rc = launch_rows<T, 12>(s, u, S, flags, a, st); break;
         default: set_error("diffusion: no strip of %d rows", s.R);
         }
-#undef NUDIM_STRIP_R
         NUDIM_TRY(rc);
         left -= rounds * s.k;
     }
     return NUDIM_OK;
 }
+
+template bool strips_fits<float>(int, int, int, double, double);
+template bool strips_fits<double>(int, int, int, double, double);
+template size_t strips_scratch<float>(int, int, int, int);
+template size_t strips_scratch<double>(int, int, int, int);
+template int strips_run<float>(float *, int, int, int, int, double, double, int, void *,
+                               cudaStream_t);
+template int strips_run<double>(double *, int, int, int, int, double, double, int, void *,
+                                cudaStream_t);
 
 }  // namespace nudim

@@ -4,7 +4,12 @@ times, every neighbour taken from what the stages produced one and two steps
 before -- restated in numpy, against the sequential Gauss-Seidel loops of
 denoise.c:320-378.  GPU: the FP32 form against the FP64 tables form at the
 edges of its strips (32 R rows), bands (384 rows), rings (P = nx or 2 K + 4)
-and sweep counts (multiples of 16 and remainders)."""
+and sweep counts (multiples of 16 and remainders); the FP64
+form bit for bit."""
+import ctypes
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -111,6 +116,94 @@ def test_strips_fp32(gpu_ctx, nudim_built, shape, nxb, it):
         if scale < 0.001:
             assert np.abs(out - ref).max() < it * 10 * 2.0 ** -24 * np.abs(v).max()
         assert rel(out, ref) < 1e-4
+
+
+INT_FLUX = r"""
+#include "intdiv.cuh"
+#include <cmath>
+extern "C" long flux_errors(const double *g, long n, float kappa)
+{
+    const double b = (double)kappa * (double)kappa;
+    nudim::DiffDiv d;
+    if (!nudim::diff_div_init(b, &d)) return -1;
+    long bad = 0;
+    for (long i = 0; i < n; i++) {
+        double f;
+        const bool ok = nudim::diff_flux_int(g[i], d, &f);
+        volatile double a = g[i] * g[i], q = a / b, s = 1.0 + q, c = 1.0 / s, r = c * g[i];
+        if (!ok) bad += std::isfinite(g[i]) && std::fabs(g[i]) < 1e100 * kappa;
+        else bad += nudim::bits_of(f) != nudim::bits_of(r);
+    }
+    return bad;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def flux_libs(tmp_path_factory):
+    """csrc/intdiv.cuh compiled for the host, the FP32 seed of its reciprocal
+    off by -2..2 units (the hardware's is within one)."""
+    d = tmp_path_factory.mktemp("intdiv")
+    (d / "f.cpp").write_text(INT_FLUX)
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nudim_gb300",
+                       "csrc")
+    libs = []
+    for k in (-2, -1, 0, 1, 2):
+        so = str(d / ("f%d.so" % k))
+        subprocess.run(["g++", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-I", inc,
+                        "-DNUDIM_SEED_SHIFT=(%d)" % k, str(d / "f.cpp"), "-o", so], check=True)
+        fn = ctypes.CDLL(so).flux_errors
+        fn.restype, fn.argtypes = ctypes.c_long, [ctypes.c_void_p, ctypes.c_long, ctypes.c_float]
+        libs.append(fn)
+    return libs
+
+
+@pytest.mark.parametrize("kappa", [0.005, 1.0, 0.5, 0.0051, 3.7, 1e-4, 0.0625, 1.9999999, 1e9])
+def test_integer_fluxes_are_the_divided_ones(flux_libs, kappa):
+    """FP64 fluxes g / (1 + g^2 / kappa^2) in integer arithmetic against the
+    host's IEEE operations, bit for bit: all scales of g / kappa, short and
+    FP32 significands (exact squares, ties), values about the rounding
+    boundaries of 1 + q, zeros, subnormals, infinities and NaN."""
+    rng = np.random.default_rng(int(kappa * 1e6) % 2 ** 31)
+    n = 100000
+    m = 1 + rng.random(n)
+    near = kappa * np.sqrt(m - 1)
+    g = np.concatenate([
+        kappa * m * 2.0 ** rng.integers(-60, 60, n), kappa * rng.standard_normal(n),
+        kappa * rng.integers(0, 4096, n) * 2.0 ** -rng.integers(0, 20, n),
+        np.float32(kappa * rng.standard_normal(n)).astype(np.float64),
+        near * (1 + rng.integers(-4, 5, n) * 2.0 ** -52),
+        rng.integers(0, 2 ** 64, n, dtype=np.uint64).view(np.float64),
+        [0.0, -0.0, 5e-324, -2e-308, np.inf, -np.inf, np.nan, kappa, -kappa]])
+    g = np.concatenate([g, -g])
+    for fn in flux_libs:
+        assert fn(g.ctypes.data, len(g), kappa) == 0
+
+
+# FP64 in strips (64 rows a band): the edges of strips, bands and rings, single
+# CTAs and clusters of 2, 4 and 8, remainders, more planes than clusters hold;
+# values the integer form does not take
+GPU_CASES64 = [((2, 1, 1), 2, 3), ((3, 2, 37), 3, 80), ((2, 64, 36), 64, 80), ((40, 65, 35), 9, 33),
+               ((3, 100, 300), 300, 47), ((76, 33, 40), 76, 17), ((160, 31, 33), 160, 9),
+               ((1, 400, 20), 20, 41)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,nxb,it", GPU_CASES64)
+def test_strips_fp64_bitwise(gpu_ctx, nudim_built, monkeypatch, shape, nxb, it):
+    v = 0.02 * np.random.default_rng(sum(shape) + it).standard_normal(shape)
+    v.flat[::7] = 0.0
+    v.flat[5::1001] *= 1e200
+    out = run(gpu_ctx, nudim_built, v, 0, 0.25, 0.005, it, nxb)
+    monkeypatch.setenv("NUDIM_DIFFUSION", "tables")
+    assert np.array_equal(out, run(gpu_ctx, nudim_built, v, 0, 0.25, 0.005, it, nxb))
+    if 2 < v.size < 100000:
+        v.flat[2] = np.nan
+        v.flat[-1] = np.inf
+        ref = run(gpu_ctx, nudim_built, v, 0, 0.25, 0.005, it, nxb)
+        monkeypatch.delenv("NUDIM_DIFFUSION")
+        out = run(gpu_ctx, nudim_built, v, 0, 0.25, 0.005, it, nxb)
+        assert np.array_equal(out, ref, equal_nan=True)
 
 
 @pytest.mark.gpu
