@@ -6,6 +6,9 @@
 // the two global sums of TV are summed in a different (tree) order.  The
 // FP32 form uses fused multiply-adds, rsqrt and fast division where noted.
 #include "engine.cuh"
+#include "intdiv.cuh"
+
+#include <cuda_pipeline.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -19,116 +22,169 @@ namespace nudim {
 //
 // One TV iteration is two launches:
 //   k_tv_grad   the gradient g of every voxel and the two global sums
-//               (sum g^2, sum of squares of the negative voxels).  A block
-//               owns a 32 x 16 (x, y) tile and a run of Z-planes; it marches
-//               along Z with three planes of the tile plus a one-cell halo in
-//               shared memory, so every voxel is read from memory about once.
-//               The halo cells hold the clamped neighbours (index -1 -> 0,
-//               n -> n-1), which are exactly the reference's boundary rules.
+//               (G = sum g^2, N = sum of squares of the negative voxels).  The four
+//               quotients of a voxel's gradient have the norms of the voxel
+//               itself and of its three upper neighbours: each voxel's norm
+//               is formed once, and the neighbours get its quotients (the
+//               same operations on the same values as four norms per voxel).  A block owns a 32 x 16 (x, y) tile and a
+//               run of Z-planes and marches along Z: per plane the tile with
+//               a one-cell halo in shared memory (clamped neighbours: index
+//               -1 -> 0, n -> n-1, the reference's boundary rules, whose
+//               differences are zero), copied in asynchronously two or three
+//               planes ahead; what the lower neighbours need goes through
+//               shared memory (FP64: the Y and X terms, FP32: the reciprocal
+//               norm), the Z part waits for the next plane; the row and
+//               column beyond the tile are formed by 48 threads more.
 //               The block that finishes last sums the per-block partials in
-//               block order (deterministic) into scal[0..1];
-//   k_tv_update u -= (lam sqrt(scal[1])) (g / sqrt(scal[0])).
+//               block order (deterministic) and leaves step[0] = sqrt(G),
+//               step[1] = lam sqrt(N) in the volume's precision (the two
+//               square roots once: in the blocks that use them they held the
+//               FP64 unit 1.6 us a block);
+//   k_tv_update u -= step[1] (g / step[0]).
+// FP64: the square root and the quotients in integer arithmetic (intdiv.cuh;
+// same bits), 18 operations of the FP64 unit a voxel left of about 110.
 constexpr int kTvTX = 32, kTvTY = 16, kTvSX = kTvTX + 2, kTvSY = kTvTY + 2;
 constexpr int kTvRows = kTvTY / 8;  // rows per thread (256 threads = 8 warps of 32 x)
 
-// Gradient of voxel (i, j, k) (denoise.c:84-122) from three tile planes:
-// p = plane clamp(i-1), q = plane i, r = plane clamp(i+1), the voxel at
-// tile cell (y, x); the reference's IEEE operations in its order (the FP64
-// form; the FP32 form runs tv_point2).
-template <typename T>
-__device__ __forceinline__ T tv_point(const T (*p)[kTvSX], const T (*q)[kTvSX],
-                                      const T (*r)[kTvSX], int y, int x, T &c)
-{
-    const T eps = (T)1e-8;
-    c = q[y][x];
-    T t1 = rn_sub(c, p[y][x]);
-    T t2 = rn_sub(c, q[y - 1][x]);
-    T t3 = rn_sub(c, q[y][x - 1]);
-    T a4 = r[y][x];
-    T t4 = rn_sub(a4, c);
-    T t5 = rn_sub(a4, r[y - 1][x]);
-    T t6 = rn_sub(a4, r[y][x - 1]);
-    T a7 = q[y + 1][x];
-    T t7 = rn_sub(a7, p[y + 1][x]);
-    T t8 = rn_sub(a7, c);
-    T t9 = rn_sub(a7, q[y + 1][x - 1]);
-    T a10 = q[y][x + 1];
-    T t10 = rn_sub(a10, p[y][x + 1]);
-    T t11 = rn_sub(a10, q[y - 1][x + 1]);
-    T t12 = rn_sub(a10, c);
-    auto nrm = [&](T x, T y, T z) {
-        return rn_sqrt(rn_add(rn_add(rn_add(eps, rn_mul(x, x)), rn_mul(y, y)), rn_mul(z, z)));
-    };
-    T g1 = rn_div(rn_add(rn_add(t1, t2), t3), nrm(t1, t2, t3));
-    T g2 = rn_div(t4, nrm(t4, t5, t6));
-    T g3 = rn_div(t8, nrm(t7, t8, t9));
-    T g4 = rn_div(t12, nrm(t10, t11, t12));
-    return rn_sub(rn_sub(rn_sub(g1, g2), g3), g4);
-}
-
-// FP32 form, two voxels at once: tile cells (y, x) and (y + 8, x), each
-// operation paired (one paired add / fused multiply-add / multiply for both
-// voxels); t / sqrt(eps + x^2 + y^2 + z^2) as t * rsqrt(...) with fused
-// multiply-adds (a few ulp per term, against one for IEEE sqrt and division;
-// the TV loop's own amplification of rounding dominates).  c returns both
-// centre values.
-__device__ __forceinline__ float2 tv_point2(const float (*p)[kTvSX], const float (*q)[kTvSX],
-                                            const float (*r)[kTvSX], int y, int x, float2 &c)
-{
-    auto ld = [&](const float (*a)[kTvSX], int yy, int xx) {
-        return make_float2(a[yy][xx], a[yy + 8][xx]);
-    };
-    auto sub = [](float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); };
-    c = ld(q, y, x);
-    const float2 t1 = sub(c, ld(p, y, x)), t2 = sub(c, ld(q, y - 1, x)),
-                 t3 = sub(c, ld(q, y, x - 1));
-    const float2 a4 = ld(r, y, x);
-    const float2 t4 = sub(a4, c), t5 = sub(a4, ld(r, y - 1, x)), t6 = sub(a4, ld(r, y, x - 1));
-    const float2 a7 = ld(q, y + 1, x);
-    const float2 t7 = sub(a7, ld(p, y + 1, x)), t8 = sub(a7, c),
-                 t9 = sub(a7, ld(q, y + 1, x - 1));
-    const float2 a10 = ld(q, y, x + 1);
-    const float2 t10 = sub(a10, ld(p, y, x + 1)), t11 = sub(a10, ld(q, y - 1, x + 1)),
-                 t12 = sub(a10, c);
-    const float2 e2 = make_float2(1e-8f, 1e-8f);
-    auto inv = [&](float2 a, float2 b, float2 d) {
-        float2 s = __ffma2_rn(d, d, __ffma2_rn(b, b, __ffma2_rn(a, a, e2)));
-        return make_float2(rsqrtf(s.x), rsqrtf(s.y));
-    };
-    const float2 h1 = __fmul2_rn(__fadd2_rn(__fadd2_rn(t1, t2), t3), inv(t1, t2, t3));
-    const float2 h2 = __fmul2_rn(t4, inv(t4, t5, t6));
-    const float2 h3 = __fmul2_rn(t8, inv(t7, t8, t9));
-    const float2 h4 = __fmul2_rn(t12, inv(t10, t11, t12));
-    return sub(sub(sub(h1, h2), h3), h4);
-}
-
-// A thread's running sum of its voxels' terms: plain in the FP64 form,
-// Neumaier-compensated in the FP32 form (a thread sums one term per plane of
-// its Z-run).
-template <typename T> struct TvAcc {
-    T s = 0, e = 0;
-    __device__ __forceinline__ void add(T x)
-    {
-        if (sizeof(T) == 8) {
-            s = rn_add(s, x);
-            return;
-        }
-        T t = rn_add(s, x);
-        e = rn_add(e, fabs(s) >= fabs(x) ? rn_add(rn_sub(s, t), x) : rn_add(rn_sub(x, t), s));
-        s = t;
-    }
-    __device__ __forceinline__ T value() const { return rn_add(s, e); }
+// A voxel's terms from its differences to the lower neighbours (denoise.c:
+// 84-122): (z + y + x) / norm and each difference / norm, norm = sqrt(1e-8 +
+// z^2 + y^2 + x^2).
+template <typename T> struct TvTerms {
+    T sum, z, y, x;
 };
 
-// The two sums: FP64 products and sums in the FP64 form; FP32 products and
+__device__ __noinline__ TvTerms<double> tv_terms_divided(double z, double y, double x)
+{
+    const double n = rn_sqrt(
+        rn_add(rn_add(rn_add(1e-8, rn_mul(z, z)), rn_mul(y, y)), rn_mul(x, x)));
+    return {rn_div(rn_add(rn_add(z, y), x), n), rn_div(z, n), rn_div(y, n), rn_div(x, n)};
+}
+
+__device__ __forceinline__ TvTerms<double> tv_terms(double z, double y, double x)
+{
+    const double s = rn_add(rn_add(rn_add(1e-8, rn_mul(z, z)), rn_mul(y, y)), rn_mul(x, x));
+    const IntDivisor n = int_sqrt(s);
+    TvTerms<double> t;
+    bool ok = (unsigned)__double2hiint(s) < 0x7ff00000u;
+    ok &= int_div(rn_add(rn_add(z, y), x), n, &t.sum);
+    ok &= int_div(z, n, &t.z);
+    ok &= int_div(y, n, &t.y);
+    ok &= int_div(x, n, &t.x);
+    if (!ok) t = tv_terms_divided(z, y, x);
+    return t;
+}
+
+// FP32: t / sqrt(...) as t * rsqrt(...) with fused multiply-adds (a few ulp per
+// term, against one for IEEE sqrt and division; the TV loop's own amplification
+// of rounding dominates).
+__device__ __forceinline__ float tv_inv(float z, float y, float x)
+{
+    return rsqrtf(__fmaf_rn(x, x, __fmaf_rn(y, y, __fmaf_rn(z, z, 1e-8f))));
+}
+
+// Quotients g / b of an update, b the gradient's norm.  FP32: from the rounded
+// reciprocal with two corrections, as the division rounds (the first brings the
+// quotient within one ulp, and from there one more correction with RN(1 / b)
+// rounds correctly: Markstein 1990; |g| is below 5, and values so small that a
+// residual underflows keep an error of an ulp).  FP64: intdiv.cuh.
+template <typename T> struct TvNorm;
+template <> struct TvNorm<float> {
+    float b, y;
+    __device__ void init(float v)
+    {
+        b = v;
+        y = v > 1e-15f && v < 1e15f ? __frcp_rn(v) : 0.f;
+    }
+    __device__ __forceinline__ float quotient(float g) const
+    {
+        if (y == 0.f) return rn_div(g, b);  // the same for the whole launch
+        float q = rn_mul(g, y);
+        q = __fmaf_rn(__fmaf_rn(-q, b, g), y, q);
+        return __fmaf_rn(__fmaf_rn(-q, b, g), y, q);
+    }
+};
+template <> struct TvNorm<double> {
+    double b;
+    IntDivisor d;
+    bool ok;
+    __device__ void init(double v)
+    {
+        b = v;
+        ok = v > 1e-300 && v < 1e300;
+        d = int_divisor(ok ? v : 1.0);
+    }
+    __device__ __forceinline__ double quotient(double g) const
+    {
+        double q;
+        if (!(int_div(g, d, &q) && ok)) q = rn_div(g, b);
+        return q;
+    }
+};
+
+// A thread's running sums of squares (gradients, negative voxels), a voxel at a
+// time: fused multiply-adds in the FP64 form, compensated in the FP32 form (a
+// thread sums two terms per plane of its Z-run; each addition's rounding error
+// exactly, by Knuth's two-sum), the two sums as a pair.
+template <typename T> struct TvAcc;
+template <> struct TvAcc<double> {
+    double g = 0, n = 0;
+    __device__ __forceinline__ void add_sq(double a, double b)
+    {
+        g = fma(a, a, g);
+        n = fma(b, b, n);
+    }
+    __device__ __forceinline__ double grad() const { return g; }
+    __device__ __forceinline__ double neg() const { return n; }
+};
+template <> struct TvAcc<float> {
+    float2 s = make_float2(0.f, 0.f), e = make_float2(0.f, 0.f);
+    __device__ __forceinline__ void add_sq(float a, float b)
+    {
+        // (a product as a fused multiply-add to -0 stays a product: the
+        // compiler would fold it into the additions)
+        const float2 m1 = make_float2(-1.f, -1.f), z = make_float2(-0.f, -0.f);
+        const float2 v = make_float2(a, b), x = __ffma2_rn(v, v, z);
+        const float2 t = __fadd2_rn(s, x), c = __ffma2_rn(m1, s, t);
+        const float2 d = __ffma2_rn(m1, c, t);
+        e = __fadd2_rn(e, __fadd2_rn(__ffma2_rn(m1, d, s), __ffma2_rn(m1, c, x)));
+        s = t;
+    }
+    __device__ __forceinline__ float grad() const { return rn_add(s.x, e.x); }
+    __device__ __forceinline__ float neg() const { return rn_add(s.y, e.y); }
+};
+
+// block_sum_t of two values with one pair of barriers (the same sums)
+template <typename T> __device__ __forceinline__ double2 block_sum2(T a, T b, double2 *sh)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    __syncthreads();
+    if (lane == 0) sh[wid] = make_double2((double)a, (double)b);
+    __syncthreads();
+    double2 v = make_double2(0, 0);
+    if (wid == 0) {
+        if (threadIdx.x < (blockDim.x + 31) >> 5) v = sh[threadIdx.x];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+            v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+        }
+    }
+    return v;
+}
+
+// The two sums: FP64 fused multiply-adds in the FP64 form; FP32 products and
 // compensated per-thread sums, FP32 warp sums and FP64 across warps and
 // blocks in the FP32 form.  Grid (x tiles, y tiles, Z-runs of zc planes);
 // 256 threads, thread (ty, tx) owns the columns (j0 + ty + 8 r, k0 + tx),
 // r < kTvRows.  done: a zeroed counter (the last block resets it).
 //
 // FUSED: the previous iteration's update is applied as the tile is read
-// (u' = u - (lam sqrt(scal_in[1])) (g_in / sqrt(scal_in[0])) on every tile
-// and halo cell, with k_tv_update's operations), the owned cells' u' are
+// (u' = u - step_in[1] (g_in / step_in[0]) on every tile and halo cell, with k_tv_update's operations), the owned cells' u' are
 // written to u_out and the gradient of u' to g: one pass reads u and g_in and
 // writes u' and g (4 values per voxel instead of the 5 of a gradient and an
 // update).  u_out and g must not alias u and g_in (other blocks still read
@@ -136,13 +192,20 @@ template <typename T> struct TvAcc {
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(256)
 k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
-          unsigned *__restrict__ done, double *__restrict__ scal, int nz, int ny, int nx,
+          unsigned *__restrict__ done, double *__restrict__ step, int nz, int ny, int nx,
           int zc, int height, int ylo, int yhi, const T *__restrict__ g_in,
-          const double *__restrict__ scal_in, double lam, T *__restrict__ u_out)
+          const double *__restrict__ step_in, double lam, T *__restrict__ u_out)
 {
     constexpr int kCells = kTvSY * kTvSX, kSlots = (kCells + 255) / 256;
-    __shared__ T pl[3][kTvSY][kTvSX];
-    __shared__ double sh[32];
+    constexpr bool FLOAT = sizeof(T) == 4;
+    constexpr int NS = FLOAT ? 4 : 3;  // planes of the ring: p, p + 1, and those in flight
+    constexpr int US = FLOAT ? 4 : 6;  // steps per loop turn (ring slot and parity constant)
+    __shared__ T pl[NS][kTvSY][kTvSX];
+    __shared__ T plg[FUSED ? NS : 1][FUSED ? kCells : 1];
+    // of the tile's voxels and of the row and column beyond, by plane parity:
+    // FP64 the Y and X terms, FP32 the reciprocal norm (in py, one wider)
+    __shared__ T py[2][kTvTY + 1][kTvTX + FLOAT], px[2][FLOAT ? 1 : kTvTY][kTvTX + 1];
+    __shared__ double2 sh[32];
     __shared__ int s_last;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int k0 = blockIdx.x * kTvTX, j0 = blockIdx.y * kTvTY;
@@ -156,119 +219,218 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
         own[r] = inb[r] && (!height || (j >= ylo && j <= yhi));
     }
     const size_t P = (size_t)ny * nx;
-    // this thread's halo-tile cells, their clamped in-plane offsets and (FUSED)
-    // whether the update applies to their row
-    int cell[kSlots];
-    size_t off[kSlots];
+    const unsigned my = (unsigned)(j0 + ty) * nx + k, my8 = my + 8u * nx;  // this thread's voxels
+    // this thread's halo-tile cells (threadIdx + 256 s), their clamped in-plane
+    // offsets and (FUSED) whether the update applies to their row
+    unsigned off[kSlots];
     bool upd[kSlots];
 #pragma unroll
     for (int s = 0; s < kSlots; s++) {
-        int c = threadIdx.x + 256 * s;
-        cell[s] = c < kCells ? c : -1;
-        int yy = c / kTvSX, xx = c - yy * kTvSX;
-        int gj = min(max(j0 + yy - 1, 0), ny - 1), gk = min(max(k0 + xx - 1, 0), nx - 1);
-        off[s] = (size_t)gj * nx + gk;
-        upd[s] = !height || (gj >= ylo && gj <= yhi);
+        const int c = threadIdx.x + 256 * s, yy = c / kTvSX, xx = c - yy * kTvSX;
+        const int gj = min(max(j0 + yy - 1, 0), ny - 1), gk = min(max(k0 + xx - 1, 0), nx - 1);
+        off[s] = (unsigned)gj * nx + gk;
+        upd[s] = c < kCells && (!height || (gj >= ylo && gj <= yhi));
     }
-    T tn = T(1), la = T(0);
-    if (FUSED) {  // the same FP64 expressions as k_tv_update
-        tn = (T)sqrt(scal_in[0]);
-        la = (T)(lam * sqrt(scal_in[1]));
-    }
-    T pre[kSlots], preg[kSlots];
-    auto fetch = [&](int plane) {
+    T la = T(0);
+    T *const cells = &pl[0][0][0] + threadIdx.x, *const gcells = &plg[0][0] + threadIdx.x;
+    // the planes of the run in order (the first and last clamped to the volume)
+    // into ring slot `sl`; past the run's end only the group's count goes on
+    const T *fu = u + (size_t)max(z0 - 1, 0) * P, *fg = g_in + (size_t)max(z0 - 1, 0) * P;
+    int fq = z0 - 1;
+    auto fetch = [&](int sl) {
+        if (fq <= z1) {
 #pragma unroll
-        for (int s = 0; s < kSlots; s++)
-            if (cell[s] >= 0) {
-                pre[s] = u[(size_t)plane * P + off[s]];
-                if (FUSED) preg[s] = g_in[(size_t)plane * P + off[s]];
-            }
-    };
-    auto store = [&](int b) {
-#pragma unroll
-        for (int s = 0; s < kSlots; s++)
-            if (cell[s] >= 0) {
-                T v = pre[s];
-                if (FUSED && upd[s]) v = rn_sub(v, rn_mul(la, rn_div(preg[s], tn)));
-                (&pl[b][0][0])[cell[s]] = v;
-            }
-    };
-    int bp = 0, bc = 1, bn = 2;
-    fetch(max(z0 - 1, 0));
-    store(bp);
-    fetch(z0);
-    store(bc);
-    fetch(min(z0 + 1, nz - 1));
-    store(bn);
-    __syncthreads();
-    TvAcc<T> ag, an;
-    for (int i = z0; i < z1; i++) {
-        if (i + 1 < z1) fetch(min(i + 2, nz - 1));  // in flight during the compute
-        if constexpr (sizeof(T) == 4 && kTvRows == 2) {
-            float2 c2;
-            const float2 g2 = tv_point2(pl[bp], pl[bc], pl[bn], ty + 1, tx + 1, c2);
-            const float gv[2] = {g2.x, g2.y}, cv[2] = {c2.x, c2.y};
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                if (FUSED && inb[r]) u_out[(size_t)i * P + (size_t)(j0 + ty + 8 * r) * nx + k] = cv[r];
-                if (own[r]) {
-                    g[(size_t)i * P + (size_t)(j0 + ty + 8 * r) * nx + k] = gv[r];
-                    ag.add(rn_mul(gv[r], gv[r]));
-                    if (cv[r] < 0.f) an.add(rn_mul(cv[r], cv[r]));
+            for (int s = 0; s < kSlots; s++)
+                if (s + 1 < kSlots || threadIdx.x < kCells - 256 * (kSlots - 1)) {
+                    __pipeline_memcpy_async(cells + sl * kCells + 256 * s, fu + off[s], sizeof(T));
+                    if (FUSED)
+                        __pipeline_memcpy_async(gcells + sl * kCells + 256 * s, fg + off[s],
+                                                sizeof(T));
                 }
+            if (fq >= 0 && fq + 1 < nz) {
+                fu += P;
+                fg += P;
+            }
+            fq++;
+        }
+        __pipeline_commit();
+    };
+    TvNorm<T> norm;
+    // u' in slot `sl`: each thread its own cells, so its own copies' arrival is
+    // all it waits for
+    auto ready = [&](int sl) {
+        if (FUSED) {
+#pragma unroll
+            for (int s = 0; s < kSlots; s++)
+                if (upd[s]) {
+                    T *v = cells + sl * kCells + 256 * s;
+                    *v = rn_sub(*v, rn_mul(la, norm.quotient(gcells[sl * kCells + 256 * s])));
+                }
+        }
+    };
+    // the voxel beyond the tile that this thread forms: row kTvTY (warp 0),
+    // column kTvTX (half of warp 1)
+    const bool extra = threadIdx.x < kTvTX + kTvTY;
+    const int ey = threadIdx.x < kTvTX ? kTvTY : threadIdx.x - kTvTX;
+    const int ex = threadIdx.x < kTvTX ? threadIdx.x : kTvTX;
+    for (int q = 0; q < NS; q++) fetch(q);  // planes z0 - 1 .. z0 + NS - 2
+    __pipeline_wait_prior(NS - 2);
+    if (FUSED) {
+        norm.init((T)step_in[0]);
+        la = (T)step_in[1];
+    }
+    ready(0);
+    ready(1);
+    __syncthreads();
+    // the plane below, and the finished plane's parts waiting for the next: its
+    // own (FP64 quotient; FP32 sum of differences and reciprocal norm), its upper
+    // neighbours' (FP64 terms; FP32 differences and reciprocal norms)
+    T below[kTvRows], cen[kTvRows], hs[kTvRows], hi[kTvRows], hy[kTvRows], hx[kTvRows];
+    T dy[kTvRows], dx[kTvRows], ebelow = T(0);
+#pragma unroll
+    for (int r = 0; r < kTvRows; r++) {
+        below[r] = pl[0][ty + 8 * r + 1][tx + 1];
+        cen[r] = hs[r] = hi[r] = hy[r] = hx[r] = dy[r] = dx[r] = T(0);
+    }
+    if (extra) ebelow = pl[0][ey + 1][ex + 1];
+    TvAcc<T> acc;
+    T *gp = g + (size_t)z0 * P, *up = FUSED ? u_out + (size_t)z0 * P : nullptr;
+    static_assert(kTvRows == 2, "two rows a thread");
+    auto finish = [&](T g0, T g1) {  // the finished plane's gradient
+        if (own[0]) gp[my] = g0;
+        if (own[1]) gp[my8] = g1;
+        gp += P;
+        acc.add_sq(own[0] ? g0 : T(0), own[0] && cen[0] < T(0) ? cen[0] : T(0));
+        acc.add_sq(own[1] ? g1 : T(0), own[1] && cen[1] < T(0) ? cen[1] : T(0));
+    };
+    // one step: plane p in slot (S + 1) mod NS
+    auto advance = [&](int p, auto sc) {
+        constexpr int S = decltype(sc)::value, sl = (S + 1) % NS, pb = S & 1;
+        const T(*q)[kTvSX] = pl[sl];
+        T c[kTvRows];
+#pragma unroll
+        for (int r = 0; r < kTvRows; r++) c[r] = q[ty + 8 * r + 1][tx + 1];
+        if constexpr (FLOAT) {
+            // two voxels at once, each operation paired.  The own quotient
+            // joins the sum unrounded, the neighbours' are rounded products
+            // (multiply-adds to -0, which the compiler does not fold on)
+            auto f2 = [](float a, float b) { return make_float2(a, b); };
+            auto prod = [&](float2 a, float2 b) { return __ffma2_rn(a, b, f2(-0.f, -0.f)); };
+            auto sub = [&](float2 a, float2 b) { return __fadd2_rn(a, f2(-b.x, -b.y)); };
+            const float2 c2 = f2(c[0], c[1]);
+            const float2 tz = sub(c2, f2(below[0], below[1]));
+            const float2 ty2 = sub(c2, f2(q[ty][tx + 1], q[ty + 8][tx + 1]));
+            const float2 tx2 = sub(c2, f2(q[ty + 1][tx], q[ty + 9][tx]));
+            const float2 s = __ffma2_rn(
+                tx2, tx2, __ffma2_rn(ty2, ty2, __ffma2_rn(tz, tz, f2(1e-8f, 1e-8f))));
+            const float2 inv = f2(rsqrtf(s.x), rsqrtf(s.y));
+            if (p > z0) {
+                // the plane below is complete with this plane's Z difference and norm
+                const float2 hz = prod(tz, inv);
+                float2 g2 = __ffma2_rn(f2(hs[0], hs[1]), f2(hi[0], hi[1]), f2(-hz.x, -hz.y));
+                g2 = sub(g2, prod(f2(dy[0], dy[1]), f2(hy[0], hy[1])));
+                g2 = sub(g2, prod(f2(dx[0], dx[1]), f2(hx[0], hx[1])));
+                finish(g2.x, g2.y);
+            }
+            const float2 h = __fadd2_rn(__fadd2_rn(tz, ty2), tx2);
+            hs[0] = h.x;
+            hs[1] = h.y;
+            hi[0] = inv.x;
+            hi[1] = inv.y;
+            py[pb][ty][tx] = inv.x;
+            py[pb][ty + 8][tx] = inv.y;
+            if (extra) {
+                const float ce = q[ey + 1][ex + 1];
+                py[pb][ey][ex] = tv_inv(rn_sub(ce, ebelow), rn_sub(ce, q[ey][ex + 1]),
+                                        rn_sub(ce, q[ey + 1][ex]));
+                ebelow = ce;
             }
         } else {
+            TvTerms<T> t[kTvRows];
+#pragma unroll
+            for (int r = 0; r < kTvRows; r++)
+                t[r] = tv_terms(rn_sub(c[r], below[r]), rn_sub(c[r], q[ty + 8 * r][tx + 1]),
+                                rn_sub(c[r], q[ty + 8 * r + 1][tx]));
+            if (p > z0)
+                finish(rn_sub(rn_sub(rn_sub(hs[0], t[0].z), hy[0]), hx[0]),
+                       rn_sub(rn_sub(rn_sub(hs[1], t[1].z), hy[1]), hx[1]));
 #pragma unroll
             for (int r = 0; r < kTvRows; r++) {
-                if (FUSED && inb[r])
-                    u_out[(size_t)i * P + (size_t)(j0 + ty + 8 * r) * nx + k] =
-                        pl[bc][ty + 8 * r + 1][tx + 1];
-                if (own[r]) {
-                    T c;
-                    T gv = tv_point<T>(pl[bp], pl[bc], pl[bn], ty + 8 * r + 1, tx + 1, c);
-                    g[(size_t)i * P + (size_t)(j0 + ty + 8 * r) * nx + k] = gv;
-                    ag.add(rn_mul(gv, gv));
-                    if (c < T(0)) an.add(rn_mul(c, c));
-                }
+                hs[r] = t[r].sum;
+                py[pb][ty + 8 * r][tx] = t[r].y;
+                px[pb][ty + 8 * r][tx] = t[r].x;
+            }
+            if (extra && p < z1) {
+                const T ce = q[ey + 1][ex + 1];
+                const TvTerms<T> te = tv_terms(rn_sub(ce, ebelow), rn_sub(ce, q[ey][ex + 1]),
+                                               rn_sub(ce, q[ey + 1][ex]));
+                if (ey == kTvTY) py[pb][kTvTY][ex] = te.y;
+                else px[pb][ey][kTvTX] = te.x;
+                ebelow = ce;
             }
         }
+        if (p == z1) return;
+#pragma unroll
+        for (int r = 0; r < kTvRows; r++) {
+            if (FUSED && inb[r]) up[r ? my8 : my] = c[r];
+            cen[r] = below[r] = c[r];
+        }
+        if (FUSED) up += P;
+        __pipeline_wait_prior(NS - 3);  // plane p + 1 is here
+        ready((sl + 1) % NS);
         __syncthreads();
-        if (i + 1 < z1) {
-            int t = bp;
-            bp = bc;
-            bc = bn;
-            bn = t;
-            store(bn);
-            __syncthreads();
+        fetch(S % NS);  // plane p + NS - 1 over plane p - 1, which has no reader left
+#pragma unroll
+        for (int r = 0; r < kTvRows; r++) {
+            hy[r] = py[pb][ty + 8 * r + 1][tx];
+            if constexpr (FLOAT) {
+                hx[r] = py[pb][ty + 8 * r][tx + 1];
+                dy[r] = rn_sub(q[ty + 8 * r + 2][tx + 1], c[r]);
+                dx[r] = rn_sub(q[ty + 8 * r + 1][tx + 2], c[r]);
+            } else {
+                hx[r] = px[pb][ty + 8 * r][tx + 1];
+            }
+        }
+    };
+    for (int p = z0; p <= z1; p += US) {
+        advance(p, std::integral_constant<int, 0>());
+        if (p + 1 <= z1) advance(p + 1, std::integral_constant<int, 1>());
+        if (p + 2 <= z1) advance(p + 2, std::integral_constant<int, 2>());
+        if (p + 3 <= z1) advance(p + 3, std::integral_constant<int, 3>());
+        if constexpr (US == 6) {
+            if (p + 4 <= z1) advance(p + 4, std::integral_constant<int, 4>());
+            if (p + 5 <= z1) advance(p + 5, std::integral_constant<int, 5>());
         }
     }
+    __pipeline_wait_prior(0);
     const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
     const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    double bg = block_sum_t<T>(ag.value(), sh);
-    double bn2 = block_sum_t<T>(an.value(), sh);
+    double2 b = block_sum2<T>(acc.grad(), acc.neg(), sh);
     if (threadIdx.x == 0) {
-        part[bid] = bg;
-        part[nblk + bid] = bn2;
+        part[bid] = b.x;
+        part[nblk + bid] = b.y;
         __threadfence();
         s_last = atomicAdd(done, 1u) == nblk - 1;
     }
     __syncthreads();
     if (!s_last) return;
     // the last block: every block's partials are visible (fence before the
-    // count); sum them in block order, the same order whichever block is last
+    // count); sum them in block order, the same order whichever block is last,
+    // and leave the step's two numbers, a square root each on two warps
     __threadfence();
-    double a = 0, b = 0;
+    b = make_double2(0, 0);
     for (int t = threadIdx.x; t < (int)nblk; t += blockDim.x) {
-        a += __ldcg(part + t);
-        b += __ldcg(part + nblk + t);
+        b.x += __ldcg(part + t);
+        b.y += __ldcg(part + nblk + t);
     }
-    a = block_sum(a, sh);
-    b = block_sum(b, sh);
+    b = block_sum2<double>(b.x, b.y, sh);
     if (threadIdx.x == 0) {
-        scal[0] = a;
-        scal[1] = b;
+        sh[0].x = b.y;
         *done = 0;
+        step[0] = (double)(T)sqrt(b.x);
     }
+    __syncthreads();
+    if (threadIdx.x == 32) step[1] = (double)(T)(lam * sqrt(sh[0].x));
 }
 
 template <typename T, int N> struct alignas(sizeof(T) * N) TvVec {
@@ -281,16 +443,12 @@ template <typename T, int N> struct alignas(sizeof(T) * N) TvVec {
 // same values).
 template <typename T, typename I, int VEC>
 __global__ void __launch_bounds__(256)
-k_tv_update(const T *u, T *u_out, const T *__restrict__ g, const double *__restrict__ scal,
-            double lam, int nz, int ny, int nx, int height, int ylo, int yhi)
+k_tv_update(const T *u, T *u_out, const T *__restrict__ g, const double *__restrict__ step,
+            int nz, int ny, int nx, int height, int ylo, int yhi)
 {
-    __shared__ T s_tn, s_la;
-    if (threadIdx.x == 0) {
-        s_tn = (T)sqrt(scal[0]);
-        s_la = (T)(lam * sqrt(scal[1]));
-    }
-    __syncthreads();
-    const T tn = s_tn, la = s_la;
+    TvNorm<T> tn;
+    tn.init((T)step[0]);
+    const T la = (T)step[1];
     const I nv = (I)nz * ny * nx / VEC, stride = (I)gridDim.x * blockDim.x;
     for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < nv; t += stride) {
         TvVec<T, VEC> x = reinterpret_cast<const TvVec<T, VEC> *>(u)[t];
@@ -301,7 +459,7 @@ k_tv_update(const T *u, T *u_out, const T *__restrict__ g, const double *__restr
                 int j = (int)(((t * VEC + e) / (I)nx) % (I)ny);
                 if (j < ylo || j > yhi) continue;
             }
-            x.v[e] = rn_sub(x.v[e], rn_mul(la, rn_div(y.v[e], tn)));
+            x.v[e] = rn_sub(x.v[e], rn_mul(la, tn.quotient(y.v[e])));
         }
         reinterpret_cast<TvVec<T, VEC> *>(u_out)[t] = x;
     }
@@ -373,11 +531,11 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     // the pointers' alignment
     auto update = [&](const T *uin, T *uout, const T *gv, const double *sc) -> int {
         if (wide(uin, uout, gv))
-            k_tv_update<T, I, W><<<(int)nuw, 256, 0, st>>>(uin, uout, gv, sc, (double)lam, nz, ny,
-                                                            nx, height, ylo, yhi);
+            k_tv_update<T, I, W><<<(int)nuw, 256, 0, st>>>(uin, uout, gv, sc, nz, ny, nx, height,
+                                                            ylo, yhi);
         else
-            k_tv_update<T, I, 1><<<(int)nu1, 256, 0, st>>>(uin, uout, gv, sc, (double)lam, nz, ny,
-                                                            nx, height, ylo, yhi);
+            k_tv_update<T, I, 1><<<(int)nu1, 256, 0, st>>>(uin, uout, gv, sc, nz, ny, nx, height,
+                                                            ylo, yhi);
         NUDIM_LAUNCH_CHECK();
         return NUDIM_OK;
     };
@@ -385,8 +543,8 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     if (!u2 || !g2 || niter < 2 || tv_unfused<T>()) {
         for (int it = 0; it < niter; it++) {
             k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc,
-                                                    height, ylo, yhi, nullptr, nullptr, 0.0,
-                                                    nullptr);
+                                                    height, ylo, yhi, nullptr, nullptr,
+                                                    (double)lam, nullptr);
             NUDIM_LAUNCH_CHECK();
             NUDIM_TRY(update(u, u, grad, scal));
         }
@@ -397,7 +555,7 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     // between (u, grad) and (u2, g2), the sums between scal[0..1] and
     // scal[2..3]), then the last update into u
     k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc, height, ylo,
-                                            yhi, nullptr, nullptr, 0.0, nullptr);
+                                            yhi, nullptr, nullptr, (double)lam, nullptr);
     NUDIM_LAUNCH_CHECK();
     T *cu = u, *cg = grad;
     double *cs = scal;

@@ -13,6 +13,7 @@
 // does), so the CPU tests hold it against the host's division.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -75,6 +76,37 @@ NUDIM_HD uint32_t seed_rcp(uint32_t f)
 #endif
 }
 
+// approximately 1 / sqrt(f) for a normal f in [1/4, 1), as FP32 bits
+NUDIM_HD uint32_t seed_rsqrt(uint32_t f)
+{
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(f)));
+    return __float_as_uint(r);
+#else
+    float x;
+    std::memcpy(&x, &f, 4);
+    x = 1.0f / std::sqrt(x);
+    uint32_t b;
+    std::memcpy(&b, &x, 4);
+#if defined(NUDIM_SEED_SHIFT)
+    b += NUDIM_SEED_SHIFT;
+#endif
+    return b;
+#endif
+}
+
+// One Newton step for 2^116 / s (s in [2^52, 2^53), y = 2^53 / s in (1, 2] as
+// y 2^63) from y1, y in 48 bits (y 2^47) within 2^-41: the residual 1 - s y1 is
+// the low 64 bits of the product, exactly.
+NUDIM_HD uint64_t recip_step(uint64_t s, uint64_t y1)
+{
+    const int64_t E = -(int64_t)(s * y1);  // 2^-100
+    const int32_t e1 = (int32_t)(E >> 29); // 2^-71
+    const int64_t c1 = ((int64_t)e1 * (int32_t)(uint32_t)(y1 >> 17)) >> 38;
+    return (y1 << 16) + (uint64_t)c1;
+}
+
 // 2^116 / s for s in (2^52, 2^53), in units of 1: y = 2^53 / s in (1, 2) as
 // y 2^63, within 3 units.  Two Newton steps: the seed's error 2^-21 goes to
 // 2^-42 (the residual 1 - d y0 from a 64 x 32-bit product) and below 2^-71
@@ -91,10 +123,7 @@ NUDIM_HD uint64_t recip63(uint64_t s)
     const int32_t e0 = (int32_t)((int64_t)(0x8000000000000000ull - p) >> 11);  // 2^-52
     const int64_t c0 = ((int64_t)e0 * (int32_t)(y0 >> 1)) >> 19;
     const uint64_t y1 = (((uint64_t)y0 << 32) + (uint64_t)c0) >> 16;  // 1.47
-    const int64_t E = -(int64_t)(s * y1);                            // 2^-100
-    const int32_t e1 = (int32_t)(E >> 29);                           // 2^-71
-    const int64_t c1 = ((int64_t)e1 * (int32_t)(uint32_t)(y1 >> 17)) >> 38;
-    return (y1 << 16) + (uint64_t)c1;
+    return recip_step(s, y1);
 }
 
 // The diffusion coefficient 1 / (1 + g^2 / b) as the reference's operations
@@ -182,6 +211,98 @@ NUDIM_HD bool diff_flux_int(double g, const DiffDiv &k, double *out)
     const uint64_t r = ((uint64_t)(uint32_t)ep << 52) + m;
     *out = double_of(eg ? (v & 0x8000000000000000ull) | r : v);
     return ok;
+}
+
+// ---------------------------------------------------------------- a / b, sqrt
+// A divisor ready for several quotients: b = n 2^(e - 52), n in [2^52, 2^53),
+// y = 2^116 / n within 4.
+struct IntDivisor {
+    uint64_t n, y;
+    int e;
+};
+
+// b positive and normal
+NUDIM_HD IntDivisor int_divisor(double b)
+{
+    const uint64_t v = bits_of(b);
+    IntDivisor d;
+    d.n = (v & 0xfffffffffffffull) | (1ull << 52);
+    d.e = (int)(v >> 52 & 0x7ff) - 1023;
+    d.y = recip63(d.n);
+    return d;
+}
+
+// RN(t / b); false where t is not finite or the quotient not a normal number
+// or zero (the caller divides).
+NUDIM_HD bool int_div(double t, const IntDivisor &d, double *out)
+{
+    const uint64_t v = bits_of(t);
+    const int et = (int)(v >> 52) & 0x7ff;
+    uint64_t m = (v & 0xfffffffffffffull) | (1ull << 52);
+    int eq = et - d.e;
+    if (m < d.n) {
+        m <<= 1;
+        eq--;
+    }
+    uint64_t q = mul_hi(m << 10, d.y) >> 10;
+    q += (int64_t)((m << 53) - (2 * q + 1) * d.n) > 0;
+    const bool zero = (v << 1) == 0;
+    const uint64_t r = ((uint64_t)(uint32_t)(eq - 1) << 52) + q;
+    *out = double_of(zero ? v : (v & 0x8000000000000000ull) | r);
+    return zero || ((unsigned)(et - 1) < 2046u && (unsigned)(eq - 1) < 2045u);
+}
+
+// RN(sqrt(s)) for a positive normal s, as a divisor.  With s = d 4^h, d in [1/4,
+// 1): y0 ~ 1 / sqrt(d) from the FP32 seed, one Newton step (within 2^-42), then
+// the square root from the 48 leading bits n1 of d y1 and the exact residual
+// d - n1^2 (within 2^-63); the last bit from the sign of 4 d - (2 n + 1)^2; and
+// the reciprocal of the rounded root by one more step.
+NUDIM_HD IntDivisor int_sqrt(double s)
+{
+    const uint64_t v = bits_of(s);
+    int e = (int)(v >> 52) - 1022;  // s = (1/2 .. 1) 2^e
+    uint64_t D = (v << 11) | (1ull << 63);
+    if (e & 1) {
+        D >>= 1;
+        e++;
+    }
+    const uint32_t dh = (uint32_t)(D >> 32);
+    // d to FP32: leading bits under the exponent of [1/2, 1) or [1/4, 1/2)
+    const uint32_t f = dh >> 31 ? 0x3f000000u + ((dh - 0x80000000u) >> 8)
+                                : 0x3e800000u + ((dh - 0x40000000u) >> 7);
+    uint32_t r = seed_rsqrt(f);
+    r = r < 0x3fffffffu ? r : 0x3fffffffu;
+    r = r > 0x3f800000u ? r : 0x3f800000u;
+    const uint32_t a0 = (r & 0x7fffffu) | 0x800000u;  // y0, 1.23
+    const uint32_t y0 = a0 << 8;                      // 1.31
+    // 1 - d y0^2 in 2^-62
+    const int64_t E = (int64_t)((1ull << 62) - mul_hi(D, ((uint64_t)a0 * a0) << 16));
+    const int32_t e0 = (int32_t)(E >> 11);  // 2^-51
+    const int64_t c0 = ((int64_t)e0 * (int32_t)(y0 >> 1)) >> 19;
+    const uint64_t y1 = ((uint64_t)y0 << 32) + (uint64_t)c0;  // 1.63
+    const uint64_t n1 = mul_hi(D, y1) >> 15;                  // sqrt(d), 48 bits
+    // d - n1^2 in 2^-96, times y / 2: in 2^-64
+    const int64_t R = (int64_t)((D << 32) - n1 * n1);
+    const int64_t cr = ((int64_t)(int32_t)(R >> 24) * (int32_t)(uint32_t)(y1 >> 33)) >> 39;
+    const uint64_t N = (n1 << 16) + (uint64_t)cr;
+    IntDivisor d;
+    d.n = N >> 11;
+    d.n += (int64_t)((D << 44) - (2 * d.n + 1) * (2 * d.n + 1)) > 0;
+    d.e = (e >> 1) - 1;
+    // a root that rounds up to the next power of two
+    const bool carry = d.n >> 53 != 0;
+    d.y = recip_step(d.n, y1 >> 16);
+    if (carry) {
+        d.n = 1ull << 52;
+        d.e++;
+        d.y = ~0ull;
+    }
+    return d;
+}
+
+NUDIM_HD double double_of(const IntDivisor &d)
+{
+    return double_of(((uint64_t)(uint32_t)(d.e + 1022) << 52) + d.n);
 }
 
 }  // namespace nudim
