@@ -42,7 +42,7 @@ namespace nudim {
 //               FP64 unit 1.6 us a block);
 //   k_tv_update u -= step[1] (g / step[0]).
 // FP64: the square root and the quotients in integer arithmetic (intdiv.cuh;
-// same bits), 18 operations of the FP64 unit a voxel left of about 110.
+// same bits), 15 operations of the FP64 unit a voxel left of about 110.
 constexpr int kTvTX = 32, kTvTY = 16, kTvSX = kTvTX + 2, kTvSY = kTvTY + 2;
 constexpr int kTvRows = kTvTY / 8;  // rows per thread (256 threads = 8 warps of 32 x)
 
@@ -62,10 +62,12 @@ __device__ __noinline__ TvTerms<double> tv_terms_divided(double z, double y, dou
 
 __device__ __forceinline__ TvTerms<double> tv_terms(double z, double y, double x)
 {
-    const double s = rn_add(rn_add(rn_add(1e-8, rn_mul(z, z)), rn_mul(y, y)), rn_mul(x, x));
-    const IntDivisor n = int_sqrt(s);
+    double z2, y2, x2;
+    bool ok = int_square(z, &z2);
+    ok &= int_square(y, &y2);
+    ok &= int_square(x, &x2);
+    const IntDivisor n = int_sqrt(rn_add(rn_add(rn_add(1e-8, z2), y2), x2));
     TvTerms<double> t;
-    bool ok = (unsigned)__double2hiint(s) < 0x7ff00000u;
     ok &= int_div(rn_add(rn_add(z, y), x), n, &t.sum);
     ok &= int_div(z, n, &t.z);
     ok &= int_div(y, n, &t.y);
@@ -87,6 +89,8 @@ __device__ __forceinline__ float tv_inv(float z, float y, float x)
 // quotient within one ulp, and from there one more correction with RN(1 / b)
 // rounds correctly: Markstein 1990; |g| is below 5, and values so small that a
 // residual underflows keep an error of an ulp).  FP64: intdiv.cuh.
+__device__ __noinline__ double tv_divided(double a, double b) { return rn_div(a, b); }
+
 template <typename T> struct TvNorm;
 template <> struct TvNorm<float> {
     float b, y;
@@ -116,22 +120,28 @@ template <> struct TvNorm<double> {
     __device__ __forceinline__ double quotient(double g) const
     {
         double q;
-        if (!(int_div(g, d, &q) && ok)) q = rn_div(g, b);
+        if (!(int_div(g, d, &q) && ok)) q = tv_divided(g, b);
         return q;
     }
 };
 
 // A thread's running sums of squares (gradients, negative voxels), a voxel at a
-// time: fused multiply-adds in the FP64 form, compensated in the FP32 form (a
-// thread sums two terms per plane of its Z-run; each addition's rounding error
+// time: plain in the FP64 form, compensated in the FP32 form (a thread sums two
+// terms per plane of its Z-run; each addition's rounding error
 // exactly, by Knuth's two-sum), the two sums as a pair.
 template <typename T> struct TvAcc;
 template <> struct TvAcc<double> {
     double g = 0, n = 0;
+    static __device__ __forceinline__ double square(double a)
+    {
+        double q;
+        if (!int_square(a, &q)) q = rn_mul(a, a);
+        return q;
+    }
     __device__ __forceinline__ void add_sq(double a, double b)
     {
-        g = fma(a, a, g);
-        n = fma(b, b, n);
+        g = rn_add(g, square(a));
+        n = rn_add(n, square(b));
     }
     __device__ __forceinline__ double grad() const { return g; }
     __device__ __forceinline__ double neg() const { return n; }
@@ -152,6 +162,10 @@ template <> struct TvAcc<float> {
     __device__ __forceinline__ float grad() const { return rn_add(s.x, e.x); }
     __device__ __forceinline__ float neg() const { return rn_add(s.y, e.y); }
 };
+
+// Blocks per SM that the cut into Z-runs (and so the order of the sums) assumes;
+// and that the kernel runs at (registers).
+template <typename T> constexpr int kTvSumBlocks = sizeof(T) == 4 ? 4 : 3;
 
 // block_sum_t of two values with one pair of barriers (the same sums)
 template <typename T> __device__ __forceinline__ double2 block_sum2(T a, T b, double2 *sh)
@@ -177,9 +191,10 @@ template <typename T> __device__ __forceinline__ double2 block_sum2(T a, T b, do
     return v;
 }
 
-// The two sums: FP64 fused multiply-adds in the FP64 form; FP32 products and
+// The two sums: FP64 products and sums in the FP64 form; FP32 products and
 // compensated per-thread sums, FP32 warp sums and FP64 across warps and
-// blocks in the FP32 form.  Grid (x tiles, y tiles, Z-runs of zc planes);
+// blocks in the FP32 form, one partial per tile and run of zc planes.  Grid (x
+// tiles, y tiles, groups of `rep` consecutive runs of `runs`);
 // 256 threads, thread (ty, tx) owns the columns (j0 + ty + 8 r, k0 + tx),
 // r < kTvRows.  done: a zeroed counter (the last block resets it).
 //
@@ -190,10 +205,10 @@ template <typename T> __device__ __forceinline__ double2 block_sum2(T a, T b, do
 // update).  u_out and g must not alias u and g_in (other blocks still read
 // their halos).
 template <typename T, bool FUSED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kTvSumBlocks<T>)
 k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
           unsigned *__restrict__ done, double *__restrict__ step, int nz, int ny, int nx,
-          int zc, int height, int ylo, int yhi, const T *__restrict__ g_in,
+          int zc, int runs, int rep, int height, int ylo, int yhi, const T *__restrict__ g_in,
           const double *__restrict__ step_in, double lam, T *__restrict__ u_out)
 {
     constexpr int kCells = kTvSY * kTvSX, kSlots = (kCells + 255) / 256;
@@ -209,7 +224,7 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
     __shared__ int s_last;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int k0 = blockIdx.x * kTvTX, j0 = blockIdx.y * kTvTY;
-    const int z0 = blockIdx.z * zc, z1 = min(nz, z0 + zc);
+    const int z0 = blockIdx.z * rep * zc, z1 = min(nz, z0 + rep * zc);
     const int k = k0 + tx;
     bool own[kTvRows], inb[kTvRows];
 #pragma unroll
@@ -294,6 +309,20 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
     }
     if (extra) ebelow = pl[0][ey + 1][ex + 1];
     TvAcc<T> acc;
+    // a finished run's partial sums
+    const unsigned nblk = gridDim.x * gridDim.y * runs;
+    int run = blockIdx.z * rep, next = z0 + zc;
+    auto emit = [&]() {
+        const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * run);
+        const double2 b = block_sum2<T>(acc.grad(), acc.neg(), sh);
+        if (threadIdx.x == 0) {
+            part[bid] = b.x;
+            part[nblk + bid] = b.y;
+        }
+        acc = TvAcc<T>();
+        run++;
+        next += zc;
+    };
     T *gp = g + (size_t)z0 * P, *up = FUSED ? u_out + (size_t)z0 * P : nullptr;
     static_assert(kTvRows == 2, "two rows a thread");
     auto finish = [&](T g0, T g1) {  // the finished plane's gradient
@@ -370,6 +399,7 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
             }
         }
         if (p == z1) return;
+        if (!FLOAT && p == next) emit();  // (FP32 blocks have one run)
 #pragma unroll
         for (int r = 0; r < kTvRows; r++) {
             if (FUSED && inb[r]) up[r ? my8 : my] = c[r];
@@ -403,14 +433,10 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
         }
     }
     __pipeline_wait_prior(0);
-    const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
-    const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    double2 b = block_sum2<T>(acc.grad(), acc.neg(), sh);
+    emit();
     if (threadIdx.x == 0) {
-        part[bid] = b.x;
-        part[nblk + bid] = b.y;
         __threadfence();
-        s_last = atomicAdd(done, 1u) == nblk - 1;
+        s_last = atomicAdd(done, 1u) == gridDim.x * gridDim.y * gridDim.z - 1;
     }
     __syncthreads();
     if (!s_last) return;
@@ -418,7 +444,7 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
     // count); sum them in block order, the same order whichever block is last,
     // and leave the step's two numbers, a square root each on two warps
     __threadfence();
-    b = make_double2(0, 0);
+    double2 b = make_double2(0, 0);
     for (int t = threadIdx.x; t < (int)nblk; t += blockDim.x) {
         b.x += __ldcg(part + t);
         b.y += __ldcg(part + nblk + t);
@@ -472,19 +498,6 @@ int tv_part_count(int nz, int ny, int nx)
     return 2 * ceil_div(nx, kTvTX) * ceil_div(ny, kTvTY) * nz + 2;
 }
 
-template <typename T> static int tv_grad_blocks_per_sm()
-{
-    static const int occ = [] {
-        int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_tv_grad<T, true>, 256, 0) !=
-                cudaSuccess ||
-            b < 1)
-            b = 1;
-        return b;
-    }();
-    return occ;
-}
-
 // Fused passes (FP32 default) or a gradient and a separate update per
 // iteration (FP64 default: the FP64 gradient is bound by the FP64 pipe, and
 // the folded update made it slower than the two launches); NUDIM_TV=
@@ -505,14 +518,21 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     int dev = 0, sms = 0;
     NUDIM_CUDA(cudaGetDevice(&dev));
     NUDIM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // Z-runs: about two resident waves of blocks, runs of at least 4 planes
-    // (each run re-reads two planes beyond its ends)
+    // Z-runs, one partial sum each: about two resident waves of blocks, runs of
+    // at least 4 planes (each run re-reads two planes beyond its ends)
     const long tiles = (long)ceil_div(nx, kTvTX) * ceil_div(ny, kTvTY);
-    const long want = 2L * sms * tv_grad_blocks_per_sm<T>();
-    const int runs = (int)std::max(1L, std::min((long)nz / 4, (long)ceil_div(want, tiles)));
-    const int zc = ceil_div(nz, runs);
-    const dim3 gg(ceil_div(nx, kTvTX), ceil_div(ny, kTvTY), ceil_div(nz, zc));
-    const long nb = (long)gg.x * gg.y * gg.z;
+    const long want = 2L * sms * kTvSumBlocks<T>;
+    const int most = (int)std::max(1L, std::min((long)nz / 4, (long)ceil_div(want, tiles)));
+    const int zc = ceil_div(nz, most), runs = ceil_div(nz, zc);
+    // FP64: as many consecutive runs per block as leave one wave (a block forms
+    // the terms of a plane beyond its last run: 128^3, two runs a block 6.4 -> 5.1
+    // ms)
+    const int rep = sizeof(T) == 8
+                        ? (int)std::max(1L, (tiles * runs + sms * kTvSumBlocks<T> - 1) /
+                                                (sms * kTvSumBlocks<T>))
+                        : 1;
+    const dim3 gg(ceil_div(nx, kTvTX), ceil_div(ny, kTvTY), ceil_div(runs, rep));
+    const long nb = tiles * runs;
     if (part_cap < 2 * nb + 1) {
         set_error("tv_run: partial buffer too small");
         return NUDIM_EINVAL;
@@ -543,7 +563,7 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     if (!u2 || !g2 || niter < 2 || tv_unfused<T>()) {
         for (int it = 0; it < niter; it++) {
             k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc,
-                                                    height, ylo, yhi, nullptr, nullptr,
+                                                    runs, rep, height, ylo, yhi, nullptr, nullptr,
                                                     (double)lam, nullptr);
             NUDIM_LAUNCH_CHECK();
             NUDIM_TRY(update(u, u, grad, scal));
@@ -554,16 +574,16 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     // previous gradient and take the next one (volumes and gradients alternate
     // between (u, grad) and (u2, g2), the sums between scal[0..1] and
     // scal[2..3]), then the last update into u
-    k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc, height, ylo,
-                                            yhi, nullptr, nullptr, (double)lam, nullptr);
+    k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc, runs, rep,
+                                            height, ylo, yhi, nullptr, nullptr, (double)lam, nullptr);
     NUDIM_LAUNCH_CHECK();
     T *cu = u, *cg = grad;
     double *cs = scal;
     for (int it = 1; it < niter; it++) {
         T *nu = cu == u ? u2 : u, *ng = cg == grad ? g2 : grad;
         double *ns = cs == scal ? scal + 2 : scal;
-        k_tv_grad<T, true><<<gg, 256, 0, st>>>(cu, ng, part, done, ns, nz, ny, nx, zc, height, ylo,
-                                               yhi, cg, cs, (double)lam, nu);
+        k_tv_grad<T, true><<<gg, 256, 0, st>>>(cu, ng, part, done, ns, nz, ny, nx, zc, runs, rep,
+                                               height, ylo, yhi, cg, cs, (double)lam, nu);
         NUDIM_LAUNCH_CHECK();
         cu = nu;
         cg = ng;

@@ -252,6 +252,23 @@ NUDIM_HD bool int_div(double t, const IntDivisor &d, double *out)
     return zero || ((unsigned)(et - 1) < 2046u && (unsigned)(eq - 1) < 2045u);
 }
 
+// RN(z z), 0 where that is below 2^-998; false where z is not finite or the
+// square near overflow.
+NUDIM_HD bool int_square(double z, double *out)
+{
+    const uint64_t v = bits_of(z);
+    const int e = (int)(v >> 52) & 0x7ff;
+    const uint64_t X = (v << 11) | (1ull << 63);
+    uint64_t h = mul_hi(X, X);  // the square's top 64 bits; the rest 0 if X is a multiple of 2^32
+    int eq = 2 * e - 1023;
+    if (h >> 63) eq++;
+    else h <<= 1;
+    uint64_t m = h >> 11;
+    m += ((uint32_t)h & 2047u) + ((uint32_t)X ? 1u : ((uint32_t)m & 1u)) > 1024u;
+    *out = double_of(e < 1023 - 499 ? 0 : ((uint64_t)(uint32_t)(eq - 1) << 52) + m);
+    return e < 1023 + 500;
+}
+
 // RN(sqrt(s)) for a positive normal s, as a divisor.  With s = d 4^h, d in [1/4,
 // 1): y0 ~ 1 / sqrt(d) from the FP32 seed, one Newton step (within 2^-42), then
 // the square root from the 48 leading bits n1 of d y1 and the exact residual
