@@ -21,7 +21,7 @@ BIN = os.path.join(PKG, "bin")
 INC = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["nfft.cu", "nfft_fused.cu", "ops.cu", "denoise.cu", "strips.cu", "api.cu", "serve.cu",
+CU_SOURCES = ["nfft.cu", "nfft_fused.cu", "toeplitz.cu", "ops.cu", "denoise.cu", "strips.cu", "api.cu", "serve.cu",
               "noalloc.cu", "project_dft.cu"]
 CXX_SOURCES = ["tables.cpp"]
 # CUDA executables beside the library (measurement helpers, no libnudim)

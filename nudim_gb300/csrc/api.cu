@@ -92,7 +92,7 @@ template <typename T> struct JobState {
     NfftDev<T> pl;
     T *img_a = nullptr, *img_b = nullptr, *grad = nullptr, *w = nullptr;
     C *data = nullptr, *y = nullptr, *r = nullptr, *v = nullptr, *z = nullptr, *p = nullptr,
-      *q = nullptr, *slices = nullptr;
+      *slices = nullptr;
     int *known = nullptr;
     void *diff = nullptr;  // diffusion scratch
     double *part = nullptr, *dots = nullptr, *tv_part = nullptr, *tv_scal = nullptr,
@@ -269,10 +269,9 @@ template <typename T> static int state_init(nudim_job *jb, JobState<T> &s)
                                    jb->stream));
     }
     if (use_toeplitz<T>(s.pl)) {
-        // CGNR's normal operator by Toeplitz embedding: T p into q; its kernel
-        // from the polar set's factors and the radial weights (the same for
-        // every line), in FP64
-        NUDIM_TRY(s.alloc(&s.q, V));
+        // CGNR's normal operator by Toeplitz embedding; its kernel from the
+        // polar set's factors and the radial weights (the same for every line),
+        // in FP64
         std::vector<double> r(np), sg(jb->A), cg(jb->A), wall, wr;
         polar_factors(jb->pad_min, jb->pad_max, jb->d.padangle, np, r.data(), sg.data(),
                       cg.data());
@@ -288,7 +287,7 @@ template <typename T> static int state_init(nudim_job *jb, JobState<T> &s)
         g.cg = cg.data();
         g.wr = jb->d.weight ? wr.data() : nullptr;
         NUDIM_TRY(s.pl.toeplitz_init(g, jb->stream));
-        s.bytes += (size_t)s.pl.nT * s.pl.nT * sizeof(cplx_t<T>);
+        s.bytes += (size_t)s.pl.nT * s.pl.nT * sizeof(T);
     }
     if (jb->d.denoise == NUDIM_DENOISE_TV) {
         NUDIM_TRY(s.alloc(&s.grad, V));
@@ -302,7 +301,7 @@ template <typename T> static int state_init(nudim_job *jb, JobState<T> &s)
         if (db) NUDIM_TRY(s.alloc(&q, db));
         s.diff = q;
     }
-    s.part_stride = cgnr_part_stride(M, (int)P2);
+    s.part_stride = std::max(cgnr_part_stride(M, (int)P2), s.pl.toeplitz ? s.pl.nT / 4 : 0);
     NUDIM_TRY(s.alloc(&s.part, (size_t)nz * s.part_stride + 2 * (size_t)nz + 2));
     NUDIM_TRY(s.alloc(&s.dots, (size_t)nz * 4));
     NUDIM_TRY(s.alloc(&s.rh, (size_t)std::max(1, jb->d.nhio + jb->d.ner)));
@@ -318,7 +317,6 @@ template <typename T> static CgnrBuffers<T> cg_bufs(JobState<T> &s)
     b.v = s.v;
     b.z = s.z;
     b.p = s.p;
-    b.q = s.q;
     b.part = s.part;
     b.part_stride = s.part_stride;
     b.dots = s.dots;
@@ -706,14 +704,14 @@ static size_t job_bytes(const nudim_job_desc *d, int A, bool both, size_t fused_
         // fused-path lists: ~11 adjoint tile entries and <= 5 trafo entries per
         // node (4-column blocks): id + 12 weights, and 3 ints + 20 weights
         b += M * (11 * (4 + 12 * sT) + 5 * (12 + 20 * sT));
-        b += nz * (size_t)cgnr_part_stride((int)M, (int)P2) * 8;
+        b += nz * (size_t)std::max(cgnr_part_stride((int)M, (int)P2), (int)n1 / 4) * 8;
         // fused-path workspace: row spectra + partials (trafo) or column
         // spectra + grid (adjoint) of one chunk of planes
         size_t plane = (np * n1 + std::max(5 * M, n1 * n1)) * sC, chunk = fused_budget / plane;
         b += (chunk < 1 ? 1 : chunk < nz ? chunk : nz) * plane;
-        // FP32 CGNR by Toeplitz embedding (grids of 256 to 1024 points): T p
-        // and the kernel's DFT
-        if (sT == 4 && n1 >= 256 && n1 <= 1024) b += V * sC + n1 * n1 * sC;
+        // FP32 CGNR by Toeplitz embedding (grids of 256 to 1024 points): the
+        // kernel's DFT
+        if (sT == 4 && n1 >= 256 && n1 <= 1024) b += n1 * n1 * sT;
         return b;
     };
     size_t b = d->precision == NUDIM_FP64 ? per(8) : per(4);

@@ -118,9 +118,7 @@ template <> constexpr int prec_of<float>() { return NUDIM_MIXED; }
 // ------------------------------------------------------------ epilogues
 enum PadMode { PM_COMPLEX = 0, PM_REAL_INIT = 1 };
 enum InterpMode { IM_PLAIN = 0, IM_RESID = 1, IM_DOTV = 2, IM_CONSTRAINT = 3 };
-// CM_TRESID / CM_TPDOT: the Toeplitz normal operator's row pass (no
-// deconvolution): z = out - T f, p = z, |z|^2 / q = T p, Re(p^H q)
-enum CropMode { CM_PLAIN = 0, CM_DOT = 1, CM_INIT = 2, CM_TRESID = 3, CM_TPDOT = 4 };
+enum CropMode { CM_PLAIN = 0, CM_DOT = 1, CM_INIT = 2 };
 
 template <typename T> struct PadArgs {
     int mode = PM_COMPLEX;
@@ -155,8 +153,7 @@ template <typename T> struct CropArgs {
     int mode = CM_PLAIN;
     cplx_t<T> *out = nullptr;
     size_t out_stride = 0;
-    cplx_t<T> *p_out = nullptr;    // CM_INIT / CM_TRESID: search direction p = z
-    const cplx_t<T> *pin = nullptr;  // CM_TPDOT: p of p^H q
+    cplx_t<T> *p_out = nullptr;    // CM_INIT: search direction p = z
     double *part = nullptr;
     int part_stride = 0;
 };
@@ -219,13 +216,11 @@ template <typename T> struct NfftDev {
     int trafo(int nplanes, const PadArgs<T> &pa, const InterpArgs<T> &ia, cudaStream_t st);
     int adjoint(int nplanes, const SpreadArgs<T> &sa, const CropArgs<T> &ca, cudaStream_t st);
 
-    // CGNR's normal operator A^H W A by Toeplitz embedding (nfft_fused.cu):
-    // khat = the nT x nT DFT of its kernel K[m] = sum_j w_j e^{2 pi i m x_j},
-    // |m| < N (computed in FP64), divided by nT^2 and laid out in the column
-    // pass's read order;
-    // ones: N0 (or N1, the larger) unit deconvolution factors for the row passes
-    C *khat = nullptr;
-    T *ones = nullptr;
+    // CGNR's normal operator A^H W A by Toeplitz embedding (toeplitz.cu): khat =
+    // the nT x nT DFT of its kernel K[m] = sum_j w_j e^{2 pi i m x_j}, |m| < N
+    // (computed in FP64; real), divided by nT^2 and laid out in the column
+    // pass's read order
+    T *khat = nullptr;
     bool toeplitz = false;
     // the circulant's size: 768 (= 24 x 32) when 2 N - 1 <= 768 < n, else the
     // NFFT grid n; twT: its twiddles e^{-2 pi i k / nT}
@@ -236,9 +231,9 @@ template <typename T> struct NfftDev {
         return fused && row_fs && N0 == N1 && n0 == n1 && (n0 == 256 || n0 == 512 || n0 == 1024);
     }
     int toeplitz_init(const PolarGeom &g, cudaStream_t st);
-    // out = T src for nplanes planes of N0 x N1 (the row pass in ca's mode;
-    // pa as for trafo: PM_COMPLEX or PM_REAL_INIT)
-    int toeplitz_apply(int nplanes, const PadArgs<T> &pa, const CropArgs<T> &ca, cudaStream_t st);
+    // the CG around it on nplanes planes (part_stride >= nT / 4)
+    int toeplitz_cg(int nplanes, C *f, const T *f_real, bool f_zero, int iters, C *z, C *p,
+                    double *part, int part_stride, double *dots, cudaStream_t st);
     int init_fused(const NfftTables &t, cudaStream_t st);
     int autotune(const NfftTables &t, cudaStream_t st);
     void release_fused();
@@ -254,11 +249,11 @@ template <typename T> struct NfftDev {
 // z/p: planes of N0*N1.  f_zero: the start value is zero (skips A f).
 // f_real: when non-null the start value is this real array (planes of
 // N0*N1) and f is overwritten with it first.
-// q: planes of N0*N1 for T p; with it and a plan whose Toeplitz operator is
-// ready, the CG runs in coefficient space (z' = z - alpha T p, v^H W v =
-// p^H T p: the same iterates as CGNR in exact arithmetic).
+// With a plan whose Toeplitz operator is ready the CG runs in coefficient space
+// (z' = z - alpha T p, v^H W v = p^H T p: the same iterates as CGNR in exact
+// arithmetic).
 template <typename T> struct CgnrBuffers {
-    cplx_t<T> *r = nullptr, *v = nullptr, *z = nullptr, *p = nullptr, *q = nullptr;
+    cplx_t<T> *r = nullptr, *v = nullptr, *z = nullptr, *p = nullptr;
     double *part = nullptr;   // nplanes * part_stride
     int part_stride = 0;
     double *dots = nullptr;   // nplanes * 4

@@ -25,16 +25,11 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "fft_regs.cuh"
 
 namespace nudim {
 
 // ================================================================ smem FFT
-template <typename T>
-__device__ __forceinline__ cplx_t<T> cmul(cplx_t<T> a, cplx_t<T> b)
-{
-    return mkc<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-
 // `cnt` FFTs of length n = 2^logn stored back to back in a; b is scratch.
 // DIR = -1 forward (e^{-2 pi i}), +1 inverse; unnormalised.  Stockham
 // autosort with radix-16 passes (a radix-8/4/2 pass last when 4 does not
@@ -48,86 +43,6 @@ __device__ __forceinline__ cplx_t<T> cmul(cplx_t<T> a, cplx_t<T> b)
 // holds the result (plain layout).
 __host__ __device__ constexpr size_t fft_buf(size_t elems) { return elems + (elems >> 4); }
 __device__ __forceinline__ int fft_pad(int i) { return i + (i >> 4); }
-
-// e^{DIR 2 pi i k / 16}, k < 16, from cos(2 pi k / 16) for k = 0..4
-template <typename T, int DIR> __device__ __forceinline__ cplx_t<T> w16(int k)
-{
-    constexpr double c[5] = {1.0, 0.92387953251128675613, 0.70710678118654752440,
-                             0.38268343236508977173, 0.0};
-    double cs, sn;
-    int q = k & 3, h = k >> 2;  // k = 4h + q: rotate (cos, sin) of q by h quarter turns
-    double cq = c[q], sq = c[4 - q];
-    switch (h & 3) {
-    case 0: cs = cq; sn = sq; break;
-    case 1: cs = -sq; sn = cq; break;
-    case 2: cs = -cq; sn = -sq; break;
-    default: cs = sq; sn = -cq; break;
-    }
-    return mkc<T>((T)cs, (T)(DIR * sn));
-}
-
-template <typename T, int DIR>
-__device__ __forceinline__ void dft2(cplx_t<T> &a0, cplx_t<T> &a1)
-{
-    cplx_t<T> t = a0;
-    a0 = mkc<T>(t.x + a1.x, t.y + a1.y);
-    a1 = mkc<T>(t.x - a1.x, t.y - a1.y);
-}
-
-template <typename T, int DIR>
-__device__ __forceinline__ void dft4(cplx_t<T> &x0, cplx_t<T> &x1, cplx_t<T> &x2, cplx_t<T> &x3)
-{
-    using C = cplx_t<T>;
-    C a0 = mkc<T>(x0.x + x2.x, x0.y + x2.y), a1 = mkc<T>(x0.x - x2.x, x0.y - x2.y);
-    C a2 = mkc<T>(x1.x + x3.x, x1.y + x3.y), a3 = mkc<T>(x1.x - x3.x, x1.y - x3.y);
-    x0 = mkc<T>(a0.x + a2.x, a0.y + a2.y);
-    x2 = mkc<T>(a0.x - a2.x, a0.y - a2.y);
-    // forward: X1 = a1 - i a3, X3 = a1 + i a3; inverse: the other way
-    if (DIR < 0) {
-        x1 = mkc<T>(a1.x + a3.y, a1.y - a3.x);
-        x3 = mkc<T>(a1.x - a3.y, a1.y + a3.x);
-    } else {
-        x1 = mkc<T>(a1.x - a3.y, a1.y + a3.x);
-        x3 = mkc<T>(a1.x + a3.y, a1.y - a3.x);
-    }
-}
-
-// R-point DFT of a[0..R) in registers.  Output X[p] is left in a[out(p)]:
-// R = 16 and 8 are split as R1 = 4 inner DFTs over m = R2 m1 + m2, the
-// twiddles e^{DIR 2 pi i m2 p1 / R} and R2-point outer DFTs, X[p1 + 4 p2] in
-// a[R2 p1 + p2].
-template <int R> __device__ __forceinline__ constexpr int dft_out(int p)
-{
-    return R == 16 ? 4 * (p & 3) + (p >> 2) : R == 8 ? 2 * (p & 3) + (p >> 2) : p;
-}
-
-template <typename T, int DIR, int R> __device__ __forceinline__ void dft_regs(cplx_t<T> *a)
-{
-    if (R == 2) {
-        dft2<T, DIR>(a[0], a[1]);
-    } else if (R == 4) {
-        dft4<T, DIR>(a[0], a[1], a[2], a[3]);
-    } else if (R == 8) {
-#pragma unroll
-        for (int m2 = 0; m2 < 2; m2++) dft4<T, DIR>(a[m2], a[2 + m2], a[4 + m2], a[6 + m2]);
-#pragma unroll
-        for (int p1 = 1; p1 < 4; p1++) a[2 * p1 + 1] = cmul<T>(a[2 * p1 + 1], w16<T, DIR>(2 * p1));
-#pragma unroll
-        for (int p1 = 0; p1 < 4; p1++) dft2<T, DIR>(a[2 * p1], a[2 * p1 + 1]);
-    } else {
-#pragma unroll
-        for (int m2 = 0; m2 < 4; m2++)
-            dft4<T, DIR>(a[m2], a[4 + m2], a[8 + m2], a[12 + m2]);
-#pragma unroll
-        for (int p1 = 1; p1 < 4; p1++)
-#pragma unroll
-            for (int m2 = 1; m2 < 4; m2++)
-                a[4 * p1 + m2] = cmul<T>(a[4 * p1 + m2], w16<T, DIR>(m2 * p1));
-#pragma unroll
-        for (int p1 = 0; p1 < 4; p1++)
-            dft4<T, DIR>(a[4 * p1], a[4 * p1 + 1], a[4 * p1 + 2], a[4 * p1 + 3]);
-    }
-}
 
 template <typename T, int DIR, int R, bool IN_PAD, bool OUT_PAD>
 __device__ __forceinline__ void fft_pass(const cplx_t<T> *__restrict__ x, cplx_t<T> *__restrict__ y,
@@ -201,128 +116,6 @@ __device__ cplx_t<T> *block_fft(cplx_t<T> *a, cplx_t<T> *b, int n, int logn, int
     return a;
 }
 
-
-// ================================================================ four-step register FFT
-// n = R1 x R2 points with one shared-memory exchange: input index l = j +
-// R2 m (j < R2, m < R1), pass 1 an R1-point DFT over m per j (registers),
-// twiddle W_n^{j k1}, exchange, pass 2 an R2-point DFT over j per k1, output
-// index k = k1 + R1 k2 (the classical four-step factorisation of the DFT).
-// R = 32 DFTs in registers split as two 16-point DFTs (dft_regs<16>) and a
-// radix-2 step with the twiddles W_32^p.
-template <typename T, int DIR> __device__ __forceinline__ cplx_t<T> w32(int p)
-{
-    // cos(2 pi p / 32), p = 0..8
-    constexpr double c[9] = {1.0,
-                             0.98078528040323044913,
-                             0.92387953251128675613,
-                             0.83146961230254523708,
-                             0.70710678118654752440,
-                             0.55557023301960222474,
-                             0.38268343236508977173,
-                             0.19509032201612826785,
-                             0.0};
-    const int q = p & 7, h = p >> 3;  // p = 8h + q: rotate by h quarter turns
-    double cs, sn;
-    const double cq = c[q], sq = c[8 - q];
-    switch (h & 3) {
-    case 0: cs = cq; sn = sq; break;
-    case 1: cs = -sq; sn = cq; break;
-    case 2: cs = -cq; sn = -sq; break;
-    default: cs = sq; sn = -cq; break;
-    }
-    return mkc<T>((T)cs, (T)(DIR * sn));
-}
-
-// W_24^p = e^{DIR 2 pi i p / 24}, p = 0..23
-template <typename T, int DIR> __device__ __forceinline__ cplx_t<T> w24(int p)
-{
-    // cos(2 pi q / 24), q = 0..6
-    constexpr double c[7] = {1.0,
-                             0.96592582628906828675,
-                             0.86602540378443864676,
-                             0.70710678118654752440,
-                             0.5,
-                             0.25881904510252076235,
-                             0.0};
-    const int q = p % 6, h = p / 6;  // p = 6h + q: rotate by h quarter turns
-    double cs, sn;
-    const double cq = c[q], sq = c[6 - q];
-    switch (h & 3) {
-    case 0: cs = cq; sn = sq; break;
-    case 1: cs = -sq; sn = cq; break;
-    case 2: cs = -cq; sn = -sq; break;
-    default: cs = sq; sn = -cq; break;
-    }
-    return mkc<T>((T)cs, (T)(DIR * sn));
-}
-
-// R-point DFT (R = 16, 24 or 32) of a[0..R) in registers; X[p] is left in
-// a[fs_out<R>(p)].  R = 24: three 8-point DFTs over a[3u + v], the twiddles
-// W_24^{v p8} and 3-point DFTs over v, X[p8 + 8q] in a[3 p8 + q].
-template <int R> __device__ __forceinline__ constexpr int fs_out(int p)
-{
-    return R == 16   ? dft_out<16>(p)
-           : R == 24 ? 3 * (p & 7) + (p >> 3)
-                     : (p < 16 ? 2 * dft_out<16>(p) : 2 * dft_out<16>(p - 16) + 1);
-}
-
-template <typename T, int DIR, int R> __device__ __forceinline__ void fs_dft(cplx_t<T> *a)
-{
-    using C = cplx_t<T>;
-    if constexpr (R == 16) {
-        dft_regs<T, DIR, 16>(a);
-    } else if constexpr (R == 24) {
-        C e[3][8];
-#pragma unroll
-        for (int v = 0; v < 3; v++)
-#pragma unroll
-            for (int u = 0; u < 8; u++) e[v][u] = a[3 * u + v];
-#pragma unroll
-        for (int v = 0; v < 3; v++) dft_regs<T, DIR, 8>(e[v]);
-        // X[p8 + 8q] = sum_v (W_24^{v p8} E_v[p8]) W_3^{v q}
-        const T h3 = (T)0.86602540378443864676;  // sqrt(3) / 2
-#pragma unroll
-        for (int p8 = 0; p8 < 8; p8++) {
-            const C x0 = e[0][dft_out<8>(p8)];
-            C x1 = e[1][dft_out<8>(p8)], x2 = e[2][dft_out<8>(p8)];
-            if (p8) {
-                x1 = cmul<T>(x1, w24<T, DIR>(p8));
-                x2 = cmul<T>(x2, w24<T, DIR>(2 * p8));
-            }
-            const C sm = mkc<T>(x1.x + x2.x, x1.y + x2.y), df = mkc<T>(x1.x - x2.x, x1.y - x2.y);
-            const C mid = mkc<T>(x0.x - (T)0.5 * sm.x, x0.y - (T)0.5 * sm.y);
-            // DIR i (sqrt(3)/2) (x1 - x2)
-            const C rot = mkc<T>(-(T)DIR * h3 * df.y, (T)DIR * h3 * df.x);
-            a[3 * p8] = mkc<T>(x0.x + sm.x, x0.y + sm.y);
-            a[3 * p8 + 1] = mkc<T>(mid.x + rot.x, mid.y + rot.y);
-            a[3 * p8 + 2] = mkc<T>(mid.x - rot.x, mid.y - rot.y);
-        }
-    } else {
-        C e[16], o[16];
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-            e[u] = a[2 * u];
-            o[u] = a[2 * u + 1];
-        }
-        dft_regs<T, DIR, 16>(e);
-        dft_regs<T, DIR, 16>(o);
-        // X[p] = E[p] + W32^p O[p], X[p + 16] = E[p] - W32^p O[p]
-#pragma unroll
-        for (int p = 0; p < 16; p++) {
-            const C ev = e[dft_out<16>(p)];
-            C ov = o[dft_out<16>(p)];
-            if (p) ov = cmul<T>(ov, w32<T, DIR>(p));
-            a[2 * dft_out<16>(p)] = mkc<T>(ev.x + ov.x, ev.y + ov.y);
-            a[2 * dft_out<16>(p) + 1] = mkc<T>(ev.x - ov.x, ev.y - ov.y);
-        }
-    }
-}
-
-template <int R1, int R2> __host__ __device__ constexpr int fs_col_stride()
-{
-    // R1 x (R2 + 1) rounded up to 4 mod 16 elements
-    return ((R1 * (R2 + 1) + 11) / 16) * 16 + 4;
-}
 
 // ================================================================ K1 row pass (trafo)
 template <typename T, int MODE>
@@ -1154,25 +947,11 @@ k_rowifft_crop_fs(const cplx_t<T> *__restrict__ Hp, int N0, int N1, const T *__r
                 if (c < N1) {
                     const C g = y[fs_out<R2>(k2)];
                     const size_t o = (size_t)gb * ca.out_stride + (size_t)a * N1 + c;
-                    if (MODE == CM_TRESID) {
-                        // z = b - T f (b in out), p = z
-                        const C bv = ca.out[o];
-                        const C z = mkc<T>(bv.x - g.x, bv.y - g.y);
-                        ca.out[o] = z;
-                        ca.p_out[o] = z;
-                        s += z.x * z.x + z.y * z.y;
-                    } else if (MODE == CM_TPDOT) {
-                        // q = T p, Re(p^H q)
-                        const C pv = ca.pin[o];
-                        ca.out[o] = g;
-                        s += pv.x * g.x + pv.y * g.y;
-                    } else {
-                        const T sc = sa * c1[c];
-                        const C z = mkc<T>(g.x * sc, g.y * sc);
-                        ca.out[o] = z;
-                        if (MODE == CM_INIT) ca.p_out[o] = z;
-                        s += z.x * z.x + z.y * z.y;
-                    }
+                    const T sc = sa * c1[c];
+                    const C z = mkc<T>(g.x * sc, g.y * sc);
+                    ca.out[o] = z;
+                    if (MODE == CM_INIT) ca.p_out[o] = z;
+                    s += z.x * z.x + z.y * z.y;
                 }
             }
         }
@@ -1242,190 +1021,6 @@ k_colifft_fs(const cplx_t<T> *__restrict__ G, int N0, int n1, const cplx_t<T> *_
             if (a < N0) Hb[(size_t)a * n1] = y[fs_out<R2>(k2)];
         }
     }
-}
-
-// ================================================================ Toeplitz column pass
-// CGNR's normal operator T = A^H W A is a convolution on the N0 x N1
-// coefficients: (T p)[k] = sum_k' K[k - k'] p[k'], K[m] = sum_j w_j
-// e^{2 pi i m x_j}, |m| < N.  Embedded in the n0 x n1 circulant (n >= 2N - 1,
-// so no wrap reaches a kept output) it is a pointwise product of DFTs: row
-// FFT of the zero-padded rows (K1' with unit factors), then per column the
-// n0-point FFT, the product with khat (the kernel's DFT / (n0 n1)) and the
-// inverse FFT, keeping the N0 rows (this kernel), then the inverse row FFT
-// with the crop (K5' with unit factors).  One CTA per (4-column block,
-// plane), R2 threads per column: pass 1 as in k_colfft_interp_fs; pass 2
-// leaves thread k1 with Y[k1 + R1 k2] for all k2, which is the first
-// (R2-point, over k2) step of the inverse four-step FFT: its outputs t2 are
-// twiddled by e^{+2 pi i k1 t2 / n0} and exchanged, and thread t2 finishes
-// with the R1-point DFT over k1 (output row t2 + R2 t1).  The exchange buffer
-// is reused for the inverse (one barrier between the last read and the first
-// write).  In place: the CTA reads and writes the same N0 x 4 values of H.
-// Three CTAs per SM (168 registers; capping the 768-point form at 128
-// registers for a fourth CTA made the passes slower, 14.4 -> 16.5 ms per
-// cfg2 iteration).
-template <typename T, int R1, int R2>
-__global__ void __launch_bounds__(4 * R2, 3)
-k_col_toeplitz(cplx_t<T> *__restrict__ H, int N0, int n1, const cplx_t<T> *__restrict__ tw0,
-               const cplx_t<T> *__restrict__ khat)
-{
-    using C = cplx_t<T>;
-    constexpr int n0 = R1 * R2, BC = 4, CS = fs_col_stride<R1, R2>(), KI = (R1 + R2 - 1) / R2;
-    static_assert(R2 * (R1 + 1) <= CS, "inverse exchange exceeds the column stride");
-    extern __shared__ __align__(16) unsigned char smraw[];
-    C *S = (C *)smraw;
-    const int cb = blockIdx.x, b = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c = lane & 3, j = warp * 8 + (lane >> 2);
-    C *Hb = H + (size_t)b * N0 * n1 + (size_t)cb * BC + c;
-    {
-        C x[R1];
-#pragma unroll
-        for (int m = 0; m < R1; m++) {
-            const int l0 = j + R2 * m;
-            const int a = (l0 < n0 / 2 ? l0 : l0 - n0) + N0 / 2;
-            x[m] = (a >= 0 && a < N0) ? Hb[(size_t)a * n1] : mkc<T>(0, 0);
-        }
-        fs_dft<T, -1, R1>(x);
-#pragma unroll
-        for (int k1 = 0; k1 < R1; k1++) {
-            C v = x[fs_out<R1>(k1)];
-            if (k1) v = cmul<T>(v, tw0[j * k1]);
-            S[c * CS + k1 * (R2 + 1) + j] = v;
-        }
-    }
-    __syncthreads();
-    C y[KI][R2];
-#pragma unroll
-    for (int i = 0; i < KI; i++)
-        if (j + R2 * i < R1)
-#pragma unroll
-            for (int jj = 0; jj < R2; jj++) y[i][jj] = S[c * CS + (j + R2 * i) * (R2 + 1) + jj];
-    __syncthreads();  // S is reused for the inverse exchange
-#pragma unroll
-    for (int i = 0; i < KI; i++) {
-        const int k1 = j + R2 * i;
-        if (k1 >= R1) break;
-        fs_dft<T, -1, R2>(y[i]);
-        C z[R2];
-        const C *kp = khat + (((size_t)cb * R2) * R1 + k1) * BC + c;
-#pragma unroll
-        for (int k2 = 0; k2 < R2; k2++)
-            z[k2] = cmul<T>(y[i][fs_out<R2>(k2)], kp[(size_t)k2 * R1 * BC]);
-        fs_dft<T, +1, R2>(z);
-#pragma unroll
-        for (int t2 = 0; t2 < R2; t2++) {
-            C v = z[fs_out<R2>(t2)];
-            if (k1 * t2) {
-                C w = tw0[k1 * t2];
-                w.y = -w.y;  // inverse: e^{+2 pi i k1 t2 / n0}
-                v = cmul<T>(v, w);
-            }
-            S[c * CS + t2 * (R1 + 1) + k1] = v;
-        }
-    }
-    __syncthreads();
-    {
-        const int t2 = j;
-        C w[R1];
-#pragma unroll
-        for (int k1 = 0; k1 < R1; k1++) w[k1] = S[c * CS + t2 * (R1 + 1) + k1];
-        fs_dft<T, +1, R1>(w);
-#pragma unroll
-        for (int t1 = 0; t1 < R1; t1++) {
-            int a = t2 + R2 * t1 + N0 / 2;
-            if (a >= n0) a -= n0;
-            if (a < N0) Hb[(size_t)a * n1] = w[fs_out<R1>(t1)];
-        }
-    }
-}
-
-// The operator's kernel in FP64 from the polar set's factored form: node
-// (a, i) = r_i (sg_a, cg_a) and weight w_i, so K[m] = sum_a G(m0 sg_a + m1
-// cg_a) with G(s) = sum_i w_i e^{2 pi i r_i s}.  G is tabulated at s_k =
-// (k - K0) delta (one thread per k, the radii summed in order) and read back
-// by 8-point Lagrange interpolation: G has at most half a turn per unit of s
-// (|r| <= 1/2), so delta = 1/32 leaves ~1e-11 relative error.
-__global__ void k_toep_gtable(const double *__restrict__ r, const double *__restrict__ w, int np,
-                              double delta, int K0, int Ns, double2 *__restrict__ G)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= Ns) return;
-    const double sv = (k - K0) * delta;
-    double re = 0, im = 0;
-    for (int i = 0; i < np; i++) {
-        double sn, cs;
-        sincospi(2.0 * r[i] * sv, &sn, &cs);
-        const double wi = w ? w[i] : 1.0;
-        re = fma(wi, cs, re);
-        im = fma(wi, sn, im);
-    }
-    G[k] = make_double2(re, im);
-}
-
-// circ[l0][l1] = K[m] for the signed indices m = (l0, l1) (mod nt) with
-// |m0| < N0, |m1| < N1, else 0; the lines summed in order.  The weights are
-// real, so K[-m] = conj(K[m]): a thread takes the m of rows l0 <= nt/2 (for
-// row 0 and row nt/2 the columns l1 <= nt/2) and also writes -m; every entry
-// is written once.
-__global__ void k_toep_circ(const double2 *__restrict__ G, double delta, int K0,
-                            const double *__restrict__ sg, const double *__restrict__ cg, int A,
-                            int N0, int N1, int nt, double2 *__restrict__ circ)
-{
-    const int h = nt / 2;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)(h + 1) * nt) return;
-    const int l0 = (int)(i / nt), l1 = (int)(i - (size_t)l0 * nt);
-    if ((l0 == 0 || l0 == h) && l1 > h) return;  // the mirror of a column l1 < h
-    const int m0 = l0 < h ? l0 : l0 - nt, m1 = l1 < h ? l1 : l1 - nt;
-    double re = 0, im = 0;
-    if (m0 > -N0 && m0 < N0 && m1 > -N1 && m1 < N1) {
-        // reciprocals of the Lagrange weights' denominators for the nodes
-        // -3..4: 1 / prod_{l != j} (j - l)
-        constexpr double rden[8] = {-1.0 / 5040, 1.0 / 720, -1.0 / 240, 1.0 / 144,
-                                    -1.0 / 144,  1.0 / 240, -1.0 / 720, 1.0 / 5040};
-        const double inv = 1.0 / delta;
-        for (int a = 0; a < A; a++) {
-            const double u = fma((double)m0, sg[a], (double)m1 * cg[a]) * inv + K0;
-            const double fu = floor(u);
-            const double t = u - fu;  // in [0, 1): nodes at t - (j - 3)
-            const int k0 = (int)fu - 3;
-            double d[8], pre[8], suf[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) d[j] = t - (j - 3);
-            pre[0] = 1.0;
-#pragma unroll
-            for (int j = 1; j < 8; j++) pre[j] = pre[j - 1] * d[j - 1];
-            suf[7] = 1.0;
-#pragma unroll
-            for (int j = 6; j >= 0; j--) suf[j] = suf[j + 1] * d[j + 1];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const double wj = pre[j] * suf[j] * rden[j];
-                const double2 gv = G[k0 + j];
-                re = fma(wj, gv.x, re);
-                im = fma(wj, gv.y, im);
-            }
-        }
-    }
-    circ[i] = make_double2(re, im);
-    const int r0 = l0 ? nt - l0 : 0, r1 = l1 ? nt - l1 : 0;  // -m (mod nt)
-    if (r0 != l0 || r1 != l1) circ[(size_t)r0 * nt + r1] = make_double2(re, -im);
-}
-
-// The circulant's DFT (row-major nt x nt, FP64) divided by nt^2, in the
-// order k_col_toeplitz<R1, R2> reads it: [block of 4 columns][k2][k1][column],
-// frequency row l0 = k1 + R1 k2.
-template <typename T>
-__global__ void k_toep_layout(const double2 *__restrict__ F, int n0, int n1, int R1, int R2,
-                              cplx_t<T> *__restrict__ khat)
-{
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n0 * n1) return;
-    const int l0 = (int)(i / n1), l1 = (int)(i - (size_t)l0 * n1);
-    const int k1 = l0 % R1, k2 = l0 / R1, cb = l1 >> 2, c = l1 & 3;
-    const double sc = 1.0 / ((double)n0 * (double)n1);
-    const double2 v = F[i];
-    khat[(((size_t)cb * R2 + k2) * R1 + k1) * 4 + c] = mkc<T>((T)(v.x * sc), (T)(v.y * sc));
 }
 
 // ================================================================ K4b column IFFT
@@ -1697,10 +1292,6 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
     NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_DOT, R1, R2>,                        \
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, L));           \
     NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_INIT, R1, R2>,                       \
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, L));           \
-    NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_TRESID, R1, R2>,                     \
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, L));           \
-    NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_TPDOT, R1, R2>,                      \
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, L))
         NUDIM_ROWFS_ATTR(32, 32, lr1);
         NUDIM_ROWFS_ATTR(32, 16, lr2);
@@ -1726,32 +1317,6 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
     NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<T, 16, 16>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, lim_col));
     // the four-step column IFFTs' exchange buffers (FP64 1024 points: 68 KB)
-    NUDIM_CUDA(cudaFuncSetAttribute(k_col_toeplitz<T, 32, 32>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(C) * 4 * fs_col_stride<32, 32>())));
-    NUDIM_CUDA(cudaFuncSetAttribute(k_col_toeplitz<T, 32, 16>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(C) * 4 * fs_col_stride<32, 16>())));
-    NUDIM_CUDA(cudaFuncSetAttribute(k_col_toeplitz<T, 16, 16>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(C) * 4 * fs_col_stride<16, 16>())));
-    NUDIM_CUDA(cudaFuncSetAttribute(k_col_toeplitz<T, 24, 32>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(C) * 4 * fs_col_stride<24, 32>())));
-    {
-        // the 768-point circulant's row passes (24 x 32)
-        const int lt = (int)(sizeof(C) * 4 * fs_row_stride<24, 32>());
-        NUDIM_CUDA(cudaFuncSetAttribute(k_rowfft_fs<T, PM_COMPLEX, 24, 32>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, lt));
-        NUDIM_CUDA(cudaFuncSetAttribute(k_rowfft_fs<T, PM_REAL_INIT, 24, 32>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, lt));
-        NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_PLAIN, 24, 32>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, lt));
-        NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_TRESID, 24, 32>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, lt));
-        NUDIM_CUDA(cudaFuncSetAttribute(k_rowifft_crop_fs<T, CM_TPDOT, 24, 32>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, lt));
-    }
     NUDIM_CUDA(cudaFuncSetAttribute(k_colifft_fs<T, 32, 32>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)(sizeof(C) * 4 * fs_col_stride<32, 32>())));
@@ -1778,12 +1343,10 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
 template <typename T> void NfftDev<T>::release_fused()
 {
     void *ptrs[] = {tw0,    tw1,  blk_off, ent,  nslots, band_off, band_node,
-                    units,  band_w, e_rb, e_cc, e_qa, e_q1, fixups, khat, ones};
-    if (twT && twT != tw0) cudaFreeAsync(twT, ast);
+                    units,  band_w, e_rb, e_cc, e_qa, e_q1, fixups, khat, twT};
     twT = nullptr;
     nT = 0;
     khat = nullptr;
-    ones = nullptr;
     toeplitz = false;
     for (void *q : ptrs)
         if (q) cudaFreeAsync(q, ast);
@@ -2089,196 +1652,6 @@ template <typename T> int NfftDev<T>::autotune(const NfftTables &t, cudaStream_t
     return NUDIM_OK;
 }
 
-// ================================================================ Toeplitz operator
-// K on the circulant in FP64 (k_toep_gtable, k_toep_circ), its nt x nt DFT
-// (cuFFT, FP64, once per plan), divided by nt^2 and laid out in the column
-// pass's read order in the plan's precision.
-template <typename T> int NfftDev<T>::toeplitz_init(const PolarGeom &g, cudaStream_t st)
-{
-    if (!toeplitz_fits()) {
-        set_error("Toeplitz operator: needs the fused four-step path on a square grid of 256, 512 "
-                  "or 1024 points");
-        return NUDIM_EINVAL;
-    }
-    if (g.A <= 0 || (size_t)g.A * N1 != (size_t)M || !g.r || !g.sg || !g.cg) {
-        set_error("Toeplitz operator: the nodes must be A lines of N1 radii");
-        return NUDIM_EINVAL;
-    }
-    if (toeplitz) return NUDIM_OK;
-    const double two_pi = 6.283185307179586;
-    // the smallest supported circulant that holds |m| < N without wrap
-    // (NUDIM_TOEPLITZ_GRID=nfft keeps the NFFT grid's size)
-    const char *eg = getenv("NUDIM_TOEPLITZ_GRID");
-    const bool small = !(eg && !strcmp(eg, "nfft"));
-    const int nt = (small && 2 * N0 - 1 <= 768 && n0 > 768) ? 768 : n0;
-    const size_t nn = (size_t)nt * nt;
-    // G's table: |s| <= |m0| + |m1| < N0 + N1
-    const double delta = 1.0 / 32;
-    const int K0 = (int)std::ceil((N0 + N1) / delta) + 8, Ns = 2 * K0 + 1;
-    std::vector<T> hones(std::max(N0, N1), T(1));
-    std::vector<C> htw(nt);
-    for (int k = 0; k < nt; k++) {
-        const double a = -two_pi * (double)k / nt;
-        htw[k] = mkc<T>((T)std::cos(a), (T)std::sin(a));
-    }
-    void *dr = nullptr, *dw = nullptr, *dsg = nullptr, *dcg = nullptr, *dG = nullptr, *dc = nullptr;
-    void *d1 = nullptr, *kh = nullptr, *dtw = nullptr;
-    // temporaries released stream-ordered after their last use; on failure
-    // the kept buffers too
-    auto done = [&](int e) {
-        for (void *q : {dr, dw, dsg, dcg, dG, dc})
-            if (q) cudaFreeAsync(q, st);
-        if (e) {
-            for (void *q : {d1, kh, dtw})
-                if (q) cudaFreeAsync(q, st);
-        }
-        return e;
-    };
-    int rc = upload_async(&dr, g.r, sizeof(double) * N1, st);
-    if (!rc && g.wr) rc = upload_async(&dw, g.wr, sizeof(double) * N1, st);
-    if (!rc) rc = upload_async(&dsg, g.sg, sizeof(double) * g.A, st);
-    if (!rc) rc = upload_async(&dcg, g.cg, sizeof(double) * g.A, st);
-    if (!rc) rc = upload_async(&d1, hones.data(), sizeof(T) * hones.size(), st);
-    if (!rc && nt != n0) rc = upload_async(&dtw, htw.data(), sizeof(C) * htw.size(), st);
-    if (rc) return done(rc);
-    if (cudaMallocAsync(&dG, sizeof(double2) * Ns, st) != cudaSuccess ||
-        cudaMallocAsync(&dc, sizeof(double2) * nn, st) != cudaSuccess ||
-        cudaMallocAsync(&kh, sizeof(C) * nn, st) != cudaSuccess) {
-        set_error("Toeplitz operator: out of device memory");
-        return done(NUDIM_ECUDA);
-    }
-    k_toep_gtable<<<(unsigned)ceil_div(Ns, 128), 128, 0, st>>>((const double *)dr,
-                                                               (const double *)dw, N1, delta, K0,
-                                                               Ns, (double2 *)dG);
-    ++g_launches;
-    k_toep_circ<<<(unsigned)ceil_div((long)(nt / 2 + 1) * nt, 128), 128, 0, st>>>(
-        (const double2 *)dG, delta, K0, (const double *)dsg, (const double *)dcg, g.A, N0, N1, nt,
-        (double2 *)dc);
-    ++g_launches;
-    if (cudaGetLastError() != cudaSuccess) {
-        set_error("Toeplitz operator: setup kernel launch failed");
-        return done(NUDIM_ECUDA);
-    }
-    cufftHandle h;
-    if ((rc = ctx_fft2d(ctx, nt, nt, 1, NUDIM_FP64, &h))) return done(rc);
-    if (cufftSetStream(h, st) != CUFFT_SUCCESS) {
-        set_error("Toeplitz operator: cufftSetStream failed");
-        return done(NUDIM_ECUDA);
-    }
-    if ((rc = fft_exec<double>(h, (double2 *)dc, CUFFT_FORWARD))) return done(rc);
-    // the column pass's four-step split of the circulant's size
-    const int R1 = nt == 256 ? 16 : nt == 768 ? 24 : 32, R2 = nt / R1;
-    k_toep_layout<T><<<(unsigned)ceil_div((long)nn, 256), 256, 0, st>>>((const double2 *)dc, nt,
-                                                                         nt, R1, R2, (C *)kh);
-    ++g_launches;
-    if (cudaGetLastError() != cudaSuccess) {
-        set_error("Toeplitz operator: setup kernel launch failed");
-        return done(NUDIM_ECUDA);
-    }
-    done(NUDIM_OK);
-    khat = (C *)kh;
-    ones = (T *)d1;
-    nT = nt;
-    twT = dtw ? (C *)dtw : tw0;
-    bytes += sizeof(C) * nn + sizeof(T) * hones.size() + (dtw ? sizeof(C) * nt : 0);
-    toeplitz = true;
-    return NUDIM_OK;
-}
-
-// out = T src over nplanes planes: row FFT of the zero-padded rows (unit
-// factors), the column pass, the inverse row FFT with the crop in ca's mode.
-// Scratch: one N0 x n1 plane of row spectra per plane of a chunk.
-template <typename T>
-int NfftDev<T>::toeplitz_apply(int nplanes, const PadArgs<T> &pa, const CropArgs<T> &ca,
-                               cudaStream_t st)
-{
-    if (!toeplitz) {
-        set_error("Toeplitz operator not initialised");
-        return NUDIM_ESTATE;
-    }
-    const int nt = nT;
-    int chunk = fused_chunk(nplanes, (size_t)N0 * nt);
-    void *wsv;
-    size_t nH = (size_t)N0 * nt * chunk;
-    NUDIM_TRY(workspace(sizeof(C) * nH, &wsv));
-    C *H = (C *)wsv;
-    const double c = sizeof(C);
-    const size_t smem_t =
-        sizeof(C) * 4 *
-        (nt == 1024  ? fs_col_stride<32, 32>()
-         : nt == 768 ? fs_col_stride<24, 32>()
-         : nt == 512 ? fs_col_stride<32, 16>()
-                     : fs_col_stride<16, 16>());
-    const size_t smem_r = nt == 768 ? sizeof(C) * 4 * fs_row_stride<24, 32>() : smem_row;
-    const int trows = nt == 768 ? 4 : rows;
-    for (int p0 = 0; p0 < nplanes; p0 += chunk) {
-        int nb = std::min(chunk, nplanes - p0);
-        {
-            ProfScope ps(ctx, PK_TOEPLITZ, st, nb * c * ((double)N0 * N1 + (double)N0 * nt));
-            dim3 g(ceil_div(N0, trows), nb);
-#define NUDIM_TROW(MD, R1, R2)                                                                   \
-    k_rowfft_fs<T, MD, R1, R2><<<g, 128, smem_r, st>>>(pa.src, pa.src_stride, N0, N1, ones, ones, \
-                                                        twT, p0, H, pa.f_init, pa.f_stride)
-            if (pa.mode == PM_COMPLEX) {
-                if (nt == 1024) NUDIM_TROW(PM_COMPLEX, 32, 32);
-                else if (nt == 768) NUDIM_TROW(PM_COMPLEX, 24, 32);
-                else if (nt == 512) NUDIM_TROW(PM_COMPLEX, 32, 16);
-                else NUDIM_TROW(PM_COMPLEX, 16, 16);
-            } else {
-                if (nt == 1024) NUDIM_TROW(PM_REAL_INIT, 32, 32);
-                else if (nt == 768) NUDIM_TROW(PM_REAL_INIT, 24, 32);
-                else if (nt == 512) NUDIM_TROW(PM_REAL_INIT, 32, 16);
-                else NUDIM_TROW(PM_REAL_INIT, 16, 16);
-            }
-#undef NUDIM_TROW
-            NUDIM_LAUNCH_CHECK();
-        }
-        {
-            // H read and written in place; khat (n0 n1 values) read per plane
-            ProfScope ps(ctx, PK_TOEPLITZ, st, nb * c * 2.0 * N0 * nt + c * (double)nt * nt);
-            if (nt == 1024)
-                k_col_toeplitz<T, 32, 32><<<dim3(nt / 4, nb), 128, smem_t, st>>>(H, N0, nt, twT,
-                                                                                  khat);
-            else if (nt == 768)
-                k_col_toeplitz<T, 24, 32><<<dim3(nt / 4, nb), 128, smem_t, st>>>(H, N0, nt, twT,
-                                                                                  khat);
-            else if (nt == 512)
-                k_col_toeplitz<T, 32, 16><<<dim3(nt / 4, nb), 64, smem_t, st>>>(H, N0, nt, twT,
-                                                                                 khat);
-            else
-                k_col_toeplitz<T, 16, 16><<<dim3(nt / 4, nb), 64, smem_t, st>>>(H, N0, nt, twT,
-                                                                                 khat);
-            NUDIM_LAUNCH_CHECK();
-        }
-        {
-            ProfScope ps(ctx, PK_TOEPLITZ, st, nb * c * ((double)N0 * nt + 2.0 * N0 * N1));
-            dim3 g(ceil_div(N0, trows), nb);
-#define NUDIM_TCROP(MD, R1, R2)                                                                  \
-    k_rowifft_crop_fs<T, MD, R1, R2><<<g, 128, smem_r, st>>>(H, N0, N1, ones, ones, twT, p0, ca)
-#define NUDIM_TCROP_N(MD)                                                                        \
-    do {                                                                                        \
-        if (nt == 1024) NUDIM_TCROP(MD, 32, 32);                                                \
-        else if (nt == 768) NUDIM_TCROP(MD, 24, 32);                                            \
-        else if (nt == 512) NUDIM_TCROP(MD, 32, 16);                                            \
-        else NUDIM_TCROP(MD, 16, 16);                                                           \
-    } while (0)
-            if (ca.mode == CM_TRESID) NUDIM_TCROP_N(CM_TRESID);
-            else if (ca.mode == CM_TPDOT) NUDIM_TCROP_N(CM_TPDOT);
-            else NUDIM_TCROP_N(CM_PLAIN);
-#undef NUDIM_TCROP_N
-#undef NUDIM_TCROP
-            NUDIM_LAUNCH_CHECK();
-        }
-    }
-    return NUDIM_OK;
-}
-
-template int NfftDev<double>::toeplitz_init(const PolarGeom &, cudaStream_t);
-template int NfftDev<float>::toeplitz_init(const PolarGeom &, cudaStream_t);
-template int NfftDev<double>::toeplitz_apply(int, const PadArgs<double> &,
-                                             const CropArgs<double> &, cudaStream_t);
-template int NfftDev<float>::toeplitz_apply(int, const PadArgs<float> &, const CropArgs<float> &,
-                                            cudaStream_t);
 template int NfftDev<double>::autotune(const NfftTables &, cudaStream_t);
 template int NfftDev<float>::autotune(const NfftTables &, cudaStream_t);
 template void NfftDev<double>::release_fused();
