@@ -53,6 +53,7 @@ struct nudim_ctx {
     double prof_bytes[nudim::PK_COUNT] = {};
     void *ws = nullptr;          // shared oversampled-grid workspace
     size_t ws_bytes = 0;
+    int sms = 0;                 // SMs of the device (ctx_sms)
     size_t grid_budget = 0;      // bytes a single NFFT pass may use for grids
     size_t fused_budget = 0;     // scratch bytes of one fused NFFT pass over a chunk of planes
     bool use_fused = true;       // NFFT path: fused (default) or cuFFT grid path
@@ -103,6 +104,7 @@ int ctx_workspace(nudim_ctx *ctx, size_t bytes, void **p);
 int upload_async(void **dst, const void *src, size_t nb, cudaStream_t st);
 int ctx_scratch(nudim_ctx *ctx, size_t bytes, double **p);
 int ctx_pool(nudim_ctx *ctx, cudaMemPool_t *pool);
+int ctx_sms(nudim_ctx *ctx);  // SMs of the context's device
 constexpr unsigned long long kPoolKeep = 512ull << 20;
 int ctx_fft2d(nudim_ctx *ctx, int n0, int n1, int batch, int prec, cufftHandle *h);
 
@@ -195,7 +197,9 @@ template <typename T> struct NfftDev {
     bool trafo_only = false;
     size_t smem_col = 0, smem_row = 0, smem_spread = 0, smem_colifft = 0;
     C *tw0 = nullptr, *tw1 = nullptr;
-    int *blk_off = nullptr, *ent = nullptr, *band_off = nullptr, *band_node = nullptr;
+    int4 *colu[2] = {nullptr, nullptr};  // trafo work units: block, first entry, end; coarse, fine
+    int ncol[2] = {0, 0};
+    int *ent = nullptr, *band_off = nullptr, *band_node = nullptr;
     T *band_w = nullptr;            // per adjoint tile entry: R row + BCa column weights
     int nE = 0;                     // trafo entries; their records (structure of arrays):
     int *e_rb = nullptr, *e_cc = nullptr;

@@ -122,6 +122,14 @@ int ctx_scratch(nudim_ctx *ctx, size_t bytes, double **p)
     return NUDIM_OK;
 }
 
+int ctx_sms(nudim_ctx *ctx)
+{
+    if (!ctx->sms &&
+        cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess)
+        ctx->sms = 152;
+    return ctx->sms;
+}
+
 int ctx_pool(nudim_ctx *ctx, cudaMemPool_t *pool)
 {
     if (!ctx->pool) {

@@ -167,6 +167,13 @@ k_rowfft(const void *__restrict__ src, size_t src_stride, int N0, int N1, int n1
     for (int idx = threadIdx.x; idx < nr * n1; idx += blockDim.x) Hb[idx] = R[idx];
 }
 
+// Entries of a trafo column CTA at most.  The polar grid's centre columns hold a
+// fifth of all nodes: as one CTA they outlast everything else.  Coarse: ten
+// sweeps of a large plane's CTA over its columns' FFTs; fine: where a launch has
+// fewer than kColFine CTAs per SM, about what the FFTs take.
+constexpr int kColEntries[2] = {8192, 512};
+constexpr int kColFine = 6;
+
 // ================================================================ K2 column pass + interpolation
 // warps per trafo column-block CTA (register room for the radix-16 FFT passes
 // and the row weights)
@@ -187,7 +194,7 @@ template <typename T> __host__ __device__ constexpr int col_warps() { return 8; 
 template <typename T>
 __global__ void __launch_bounds__(32 * col_warps<T>(), sizeof(T) == 4 ? NUDIM_COL_MINB : 1)
 k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int n1, int BC,
-                const cplx_t<T> *__restrict__ tw0, const int *__restrict__ blk_off,
+                const cplx_t<T> *__restrict__ tw0, const int4 *__restrict__ units,
                 const int *__restrict__ ent, const int *__restrict__ e_rb,
                 const int *__restrict__ e_cc, const T *__restrict__ e_qa,
                 const T *__restrict__ e_q1, int nE, int M, int smax,
@@ -196,7 +203,8 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
     using C = cplx_t<T>;
     extern __shared__ __align__(16) unsigned char smraw[];
     C *A = (C *)smraw, *B = A + fft_buf((size_t)BC * n0);
-    int cb = blockIdx.x, b = blockIdx.y;
+    const int4 un = units[blockIdx.x];
+    int cb = un.x, b = blockIdx.y;
     const C *Hb = H + (size_t)b * N0 * n1 + (size_t)cb * BC;
     // rows a of H land at l0 = (a - N0/2) mod n0; the other rows are zero.
     // Eight loads per thread in flight before the shared-memory stores.
@@ -224,7 +232,7 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
     }
     __syncthreads();
     const C *G = block_fft<T, -1>(A, B, n0, logn0, BC, tw0);
-    const int beg = blk_off[cb], end = blk_off[cb + 1];
+    const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
@@ -278,7 +286,7 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
 template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(32 * col_warps<T>(), sizeof(T) == 4 ? NUDIM_COL_MINB : 1)
 k_colfft_interp_fs(const cplx_t<T> *__restrict__ H, int N0, int n1,
-                   const cplx_t<T> *__restrict__ tw0, const int *__restrict__ blk_off,
+                   const cplx_t<T> *__restrict__ tw0, const int4 *__restrict__ units,
                    const int *__restrict__ ent, const int *__restrict__ e_rb,
                    const int *__restrict__ e_cc, const T *__restrict__ e_qa,
                    const T *__restrict__ e_q1, int nE, int M, int smax,
@@ -288,7 +296,8 @@ k_colfft_interp_fs(const cplx_t<T> *__restrict__ H, int N0, int n1,
     constexpr int n0 = R1 * R2, BC = 4, GS = n0 + 8, CS = fs_col_stride<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
     C *Gs = (C *)smraw, *S = Gs + BC * GS;
-    const int cb = blockIdx.x, b = blockIdx.y;
+    const int4 un = units[blockIdx.x];
+    const int cb = un.x, b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool fft = threadIdx.x < 4 * R2;
     const int c = lane & 3, j = warp * 8 + (lane >> 2);
@@ -321,7 +330,7 @@ k_colfft_interp_fs(const cplx_t<T> *__restrict__ H, int N0, int n1,
         }
     }
     __syncthreads();
-    const int beg = blk_off[cb], end = blk_off[cb + 1];
+    const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
@@ -383,7 +392,7 @@ template <int R1, int R2> __host__ __device__ constexpr int fs2_gs()
 template <int R1, int R2>
 __global__ void __launch_bounds__(256, 3)
 k_colfft_interp_fs2(const float2 *__restrict__ H, int N0, int n1, int nb_planes,
-                    const float2 *__restrict__ tw0, const int *__restrict__ blk_off,
+                    const float2 *__restrict__ tw0, const int4 *__restrict__ units,
                     const int *__restrict__ ent, const int *__restrict__ e_rb,
                     const int *__restrict__ e_cc, const float *__restrict__ e_qa,
                     const float *__restrict__ e_q1, int nE, int M, int smax,
@@ -393,7 +402,8 @@ k_colfft_interp_fs2(const float2 *__restrict__ H, int N0, int n1, int nb_planes,
     constexpr int n0 = R1 * R2, BC = 4, GS = fs2_gs<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
     C *Gs = (C *)smraw;  // [plane 0..1][column][GS]
-    const int cb = blockIdx.x, pb = blockIdx.y * 2;
+    const int4 un = units[blockIdx.x];
+    const int cb = un.x, pb = blockIdx.y * 2;
     const bool two = pb + 1 < nb_planes;
     const int pp = threadIdx.x >> 7, t = threadIdx.x & 127;
     const int lane = t & 31, warp = t >> 5;
@@ -444,7 +454,7 @@ k_colfft_interp_fs2(const float2 *__restrict__ H, int N0, int n1, int nb_planes,
         }
     }
     __syncthreads();
-    const int beg = blk_off[cb], end = blk_off[cb + 1];
+    const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
@@ -495,7 +505,7 @@ template <int R1, int R2> __host__ __device__ constexpr int fs8_gs()
 template <int R1, int R2>
 __global__ void __launch_bounds__(256, 3)
 k_colfft_interp_fs8(const float2 *__restrict__ H, int N0, int n1,
-                    const float2 *__restrict__ tw0, const int *__restrict__ blk_off,
+                    const float2 *__restrict__ tw0, const int4 *__restrict__ units,
                     const int *__restrict__ ent, const int *__restrict__ e_rb,
                     const int *__restrict__ e_cc, const float *__restrict__ e_qa,
                     const float *__restrict__ e_q1, int nE, int M, int smax,
@@ -505,7 +515,8 @@ k_colfft_interp_fs8(const float2 *__restrict__ H, int N0, int n1,
     constexpr int n0 = R1 * R2, BC = 8, GS = fs8_gs<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
     C *Gs = (C *)smraw;  // [column][GS]
-    const int cb = blockIdx.x, b = blockIdx.y;
+    const int4 un = units[blockIdx.x];
+    const int cb = un.x, b = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = lane & 7, j = warp * 4 + (lane >> 3);
     const bool fft = j < R2;
@@ -548,7 +559,7 @@ k_colfft_interp_fs8(const float2 *__restrict__ H, int N0, int n1,
         }
     }
     __syncthreads();
-    const int beg = blk_off[cb], end = blk_off[cb + 1];
+    const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
@@ -681,7 +692,10 @@ struct Kahan2 {
 // its warps share them out through a shared counter.  No grid point has two
 // writers and every sum has a fixed order: the results are deterministic.
 constexpr int kGatherWarps = 8;
-constexpr int kGatherUnitsPerCta = 16;
+// units per CTA, and where a launch has fewer than kGatherFine CTAs per SM of
+// them: one per warp (the longest ones bound such a launch), on fewer planes at
+// a time
+constexpr int kGatherUnitsPerCta = 16, kGatherFine = 4;
 constexpr int kGatherMaxEntries = 128;
 
 // node values of a stage: row stride in complex elements (padded so the
@@ -692,28 +706,24 @@ template <typename T, int P> __host__ __device__ constexpr size_t gather_stage_b
     return 32 * ((size_t)W * sizeof(T) + (size_t)gather_fs_stride<P>() * sizeof(cplx_t<T>));
 }
 
+// The units of a CTA for its group's np <= P planes from pb on.
 template <typename T, bool WEIGHTED, int P>
-__global__ void __launch_bounds__(32 * kGatherWarps, 3)
-k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits,
-                const int *__restrict__ band_node, const T *__restrict__ band_w, int nbands,
-                int n0, int n1, int BC, int nb_planes, int plane0, cplx_t<T> *__restrict__ G,
-                cplx_t<T> *__restrict__ part)
+__device__ __forceinline__ void
+gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, int t1, int &next_tile,
+             const int *__restrict__ band_node, const T *__restrict__ band_w, int nbands, int n0,
+             int n1, int BC, int nb_planes, int plane0, int pb, int np, unsigned char *smraw,
+             cplx_t<T> *__restrict__ G, cplx_t<T> *__restrict__ part)
 {
     using C = cplx_t<T>;
     constexpr int FS = gather_fs_stride<P>();
-    extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ int next_tile;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int R = 32 / BC, W = R + BC, nblk = n1 / BC;
+    const int R = 32 / BC, W = R + BC;
     T *ws = (T *)(smraw + warp * gather_stage_bytes<T, P>(W));  // [32][W] weights
     C *fs = (C *)(ws + 32 * W);                                 // [32][FS] node values
-    const int pb = blockIdx.y * P, np = min(P, nb_planes - pb);
-    const int t0 = blockIdx.x * kGatherUnitsPerCta;
-    const int t1 = min(nunits, t0 + kGatherUnitsPerCta);
-    if (threadIdx.x == 0) next_tile = t0 + kGatherWarps;
-    __syncthreads();
     const int rr = lane / BC, cc = lane - rr * BC;
     const int wv16 = W * (int)sizeof(T) / 16;  // 16-byte vectors of an entry's weights
+    const C *f0 = sa.f + (size_t)(plane0 + pb) * sa.f_stride;
+    C *G0 = G + (size_t)pb * n0 * n1;
     int it = t0 + warp;
     while (it < t1) {
         const int4 un = units[it];  // tile, first entry, end, partial slot (0: G)
@@ -734,15 +744,17 @@ k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits,
                 float4 *dst = reinterpret_cast<float4 *>(ws + lane * W);
                 for (int q = 0; q < wv16; q++) dst[q] = src[q];
                 const T wv = WEIGHTED ? sa.w[j] : T(1);
+                const C *fp = f0 + j;
+                C fv[P];
 #pragma unroll
                 for (int p = 0; p < P; p++) {
-                    C fv = mkc<T>(0, 0);
-                    if (p < np) {
-                        fv = sa.f[(size_t)(plane0 + pb + p) * sa.f_stride + j];
-                        if (WEIGHTED) fv = mkc<T>(wv * fv.x, wv * fv.y);
-                    }
-                    fs[lane * FS + p] = fv;
+                    fv[p] = mkc<T>(0, 0);
+                    if (p < np) fv[p] = *fp;
+                    fp += sa.f_stride;
                 }
+#pragma unroll
+                for (int p = 0; p < P; p++)
+                    fs[lane * FS + p] = WEIGHTED ? mkc<T>(wv * fv[p].x, wv * fv[p].y) : fv[p];
             }
             __syncwarp();
             if constexpr (sizeof(T) == 4) {
@@ -768,8 +780,14 @@ k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits,
                         }
                     }
                 }
+                // (the first chunk's addition to zero is its own sum)
+                if (base == beg) {
 #pragma unroll
-                for (int p = 0; p < P; p++) ks[p].add(bs[p]);
+                    for (int p = 0; p < P; p++) ks[p].s = bs[p];
+                } else {
+#pragma unroll
+                    for (int p = 0; p < P; p++) ks[p].add(bs[p]);
+                }
             } else {
                 // FP64: the point's weight once per entry, then one fused
                 // multiply-add per plane and component (the FP64 pipe is
@@ -787,25 +805,51 @@ k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits,
             __syncwarp();  // the stage is refilled by the next chunk
         }
         const int b = tile / nbands, v = tile - b * nbands;
+        C *out = un.w == 0 ? G0 + ((size_t)b * n0 + (size_t)v * R) * BC + lane
+                           : part + ((size_t)(un.w - 1) * nb_planes + pb) * 32 + lane;
+        const size_t step = un.w == 0 ? (size_t)n0 * n1 : 32;
 #pragma unroll
         for (int p = 0; p < P; p++) {
-            if (p < np) {
-                if (sizeof(T) == 4) {
-                    const float2 v = ks[p].value();
-                    ar[p] = (T)v.x;
-                    ai[p] = (T)v.y;
-                }
-                const C val = mkc<T>(ar[p], ai[p]);
-                if (un.w == 0)
-                    G[(((size_t)(pb + p) * nblk + b) * n0 + (size_t)v * R) * BC + lane] = val;
-                else
-                    part[(((size_t)(un.w - 1) * nb_planes) + pb + p) * 32 + lane] = val;
+            if (sizeof(T) == 4) {
+                const float2 v = ks[p].value();
+                ar[p] = (T)v.x;
+                ai[p] = (T)v.y;
             }
+            if (p < np) *out = mkc<T>(ar[p], ai[p]);
+            out += step;
         }
         int nt = 0;
         if (lane == 0) nt = atomicAdd(&next_tile, 1);
         it = __shfl_sync(0xffffffffu, nt, 0);
     }
+}
+
+// A last group of at most half the planes takes the loop for so many.
+template <typename T, bool WEIGHTED, int P>
+__global__ void __launch_bounds__(32 * kGatherWarps, 3)
+k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits, int upc,
+                const int *__restrict__ band_node, const T *__restrict__ band_w, int nbands,
+                int n0, int n1, int BC, int nb_planes, int plane0, cplx_t<T> *__restrict__ G,
+                cplx_t<T> *__restrict__ part)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ int next_tile;
+    const int pb = blockIdx.y * P, np = min(P, nb_planes - pb);
+    const int t0 = blockIdx.x * upc;
+    const int t1 = min(nunits, t0 + upc);
+    if (threadIdx.x == 0) next_tile = t0 + kGatherWarps;
+    __syncthreads();
+#define NUDIM_UNITS(PP)                                                                          \
+    gather_units<T, WEIGHTED, PP>(sa, units, t0, t1, next_tile, band_node, band_w, nbands, n0,   \
+                                  n1, BC, nb_planes, plane0, pb, np, smraw, G, part)
+    if constexpr (P >= 8) {
+        if (np <= 2) NUDIM_UNITS(2);
+        else if (np <= 4) NUDIM_UNITS(4);
+        else NUDIM_UNITS(P);
+    } else {
+        NUDIM_UNITS(P);
+    }
+#undef NUDIM_UNITS
 }
 
 // The tiles whose lists were split into several ranges: their grid points
@@ -1244,7 +1288,23 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
     };
     NUDIM_TRY(up((void **)&tw0, t0.data(), sizeof(T) * t0.size()));
     NUDIM_TRY(up((void **)&tw1, t1.data(), sizeof(T) * t1.size()));
-    NUDIM_TRY(up((void **)&blk_off, L.blk_off.data(), sizeof(int) * L.blk_off.size()));
+    // trafo work units: a block's entries in ranges of at most kColEntries
+    // (nothing splits the FFT: every range's CTA does the block's columns), the
+    // fine ranges for launches that leave SMs idle; longest first
+    for (int f = 0; f < 2; f++) {
+        std::vector<int4> cu;
+        for (int b = 0; b < nblk; b++) {
+            const int b0 = L.blk_off[b], len = L.blk_off[b + 1] - b0;
+            const int nr = std::max(1, ceil_div(len, kColEntries[f]));
+            for (int r = 0; r < nr; r++)
+                cu.push_back(make_int4(b, b0 + (int)((long)len * r / nr),
+                                       b0 + (int)((long)len * (r + 1) / nr), 0));
+        }
+        std::stable_sort(cu.begin(), cu.end(),
+                         [](const int4 &a, const int4 &b) { return a.z - a.y > b.z - b.y; });
+        ncol[f] = (int)cu.size();
+        NUDIM_TRY(up((void **)&colu[f], cu.data(), sizeof(int4) * cu.size()));
+    }
     NUDIM_TRY(up((void **)&ent, L.ent.data(), sizeof(int) * L.ent.size()));
     NUDIM_TRY(up((void **)&nslots, L.nslots.data(), L.nslots.size()));
     nE = (int)L.ent.size();
@@ -1342,7 +1402,7 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
 
 template <typename T> void NfftDev<T>::release_fused()
 {
-    void *ptrs[] = {tw0,    tw1,  blk_off, ent,  nslots, band_off, band_node,
+    void *ptrs[] = {tw0,    tw1,  colu[0], colu[1], ent,  nslots, band_off, band_node,
                     units,  band_w, e_rb, e_cc, e_qa, e_q1, fixups, khat, twT};
     twT = nullptr;
     nT = 0;
@@ -1351,7 +1411,8 @@ template <typename T> void NfftDev<T>::release_fused()
     for (void *q : ptrs)
         if (q) cudaFreeAsync(q, ast);
     tw0 = tw1 = nullptr;
-    blk_off = ent = band_off = band_node = e_rb = e_cc = nullptr;
+    colu[0] = colu[1] = nullptr;
+    ent = band_off = band_node = e_rb = e_cc = nullptr;
     units = fixups = nullptr;
     band_w = e_qa = e_q1 = nullptr;
     nslots = nullptr;
@@ -1419,19 +1480,22 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
         {
             ProfScope ps(ctx, PK_INTERP, st,
                          tab + nb * c * ((double)N0 * n1 + (double)smax * M));
+            const int f = ctx_sms(ctx) * kColFine > nblk * nb;
+            const int4 *cu = colu[f];
+            const int nc = ncol[f];
             // one radix-16 butterfly per thread: 64 threads per column
             const int thr = std::min(32 * col_warps<T>(), std::max(64, 64 * BC));
 #define NUDIM_COLFS(R1, R2)                                                                      \
-    k_colfft_interp_fs<T, R1, R2><<<dim3(nblk, nb), thr, smem_colfs_of<T>(R1, R2), st>>>(             \
-        H, N0, n1, tw0, blk_off, ent, e_rb, e_cc, e_qa, e_q1, nE, M, smax, P)
+    k_colfft_interp_fs<T, R1, R2><<<dim3(nc, nb), thr, smem_colfs_of<T>(R1, R2), st>>>(             \
+        H, N0, n1, tw0, cu, ent, e_rb, e_cc, e_qa, e_q1, nE, M, smax, P)
 #define NUDIM_COLFS2(R1, R2)                                                                     \
-    k_colfft_interp_fs2<R1, R2><<<dim3(nblk, ceil_div(nb, 2)), 256,                             \
+    k_colfft_interp_fs2<R1, R2><<<dim3(nc, ceil_div(nb, 2)), 256,                             \
                                   sizeof(float2) * 2 * 4 * fs2_gs<R1, R2>(), st>>>(             \
-        (const float2 *)H, N0, n1, nb, (const float2 *)tw0, blk_off, ent, e_rb, e_cc,            \
+        (const float2 *)H, N0, n1, nb, (const float2 *)tw0, cu, ent, e_rb, e_cc,            \
         (const float *)e_qa, (const float *)e_q1, nE, M, smax, (float2 *)P)
 #define NUDIM_COLFS8(R1, R2)                                                                     \
-    k_colfft_interp_fs8<R1, R2><<<dim3(nblk, nb), 256, sizeof(float2) * 8 * fs8_gs<R1, R2>(),    \
-                                  st>>>((const float2 *)H, N0, n1, (const float2 *)tw0, blk_off, \
+    k_colfft_interp_fs8<R1, R2><<<dim3(nc, nb), 256, sizeof(float2) * 8 * fs8_gs<R1, R2>(),    \
+                                  st>>>((const float2 *)H, N0, n1, (const float2 *)tw0, cu,      \
                                         ent, e_rb, e_cc, (const float *)e_qa,                   \
                                         (const float *)e_q1, nE, M, smax, (float2 *)P)
             if (sizeof(T) == 4 && BC == 8 && n0 == 1024) NUDIM_COLFS8(32, 32);
@@ -1444,8 +1508,8 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             else if (BC == 4 && n0 == 512) NUDIM_COLFS(32, 16);
             else if (BC == 4 && n0 == 256) NUDIM_COLFS(16, 16);
             else
-                k_colfft_interp<T><<<dim3(nblk, nb), thr, smem_col, st>>>(
-                    H, N0, n0, logn0, n1, BC, tw0, blk_off, ent, e_rb, e_cc, e_qa, e_q1, nE, M,
+                k_colfft_interp<T><<<dim3(nc, nb), thr, smem_col, st>>>(
+                    H, N0, n0, logn0, n1, BC, tw0, cu, ent, e_rb, e_cc, e_qa, e_q1, nE, M,
                     smax, P);
 #undef NUDIM_COLFS
 #undef NUDIM_COLFS2
@@ -1489,21 +1553,26 @@ int NfftDev<T>::adjoint_fused(int nplanes, const SpreadArgs<T> &sa, const CropAr
         int nb = std::min(chunk, nplanes - p0);
         {
             ProfScope ps(ctx, PK_SPREAD, st, tab + nb * c * ((double)M + (double)n0 * n1));
-            dim3 g(ceil_div(nunits, kGatherUnitsPerCta), ceil_div(nb, Pa));
+            const int few = kGatherFine * ctx_sms(ctx);
+            int Pl = Pa, upc = kGatherUnitsPerCta;
+            auto ctas = [&]() { return ceil_div(nunits, upc) * ceil_div(nb, Pl); };
+            if (ctas() < few) upc = kGatherWarps;
+            while (Pl > 2 && ctas() < few) Pl /= 2;
+            dim3 g(ceil_div(nunits, upc), ceil_div(nb, Pl));
             const int thr = 32 * kGatherWarps;
 #define NUDIM_GATHER(WT, PP)                                                                    \
-    k_spread_gather<T, WT, PP><<<g, thr, smem_spread, st>>>(sa, units, nunits, band_node,       \
+    k_spread_gather<T, WT, PP><<<g, thr, smem_spread, st>>>(sa, units, nunits, upc, band_node,  \
                                                             band_w, nbands, n0, n1, BCa, nb,    \
                                                             p0, G, part)
             if (sa.w) {
-                if (Pa == 8) NUDIM_GATHER(true, 8);
-                else if (Pa == 4) NUDIM_GATHER(true, 4);
-                else if (Pa == 2) NUDIM_GATHER(true, 2);
+                if (Pl == 8) NUDIM_GATHER(true, 8);
+                else if (Pl == 4) NUDIM_GATHER(true, 4);
+                else if (Pl == 2) NUDIM_GATHER(true, 2);
                 else NUDIM_GATHER(true, 1);
             } else {
-                if (Pa == 8) NUDIM_GATHER(false, 8);
-                else if (Pa == 4) NUDIM_GATHER(false, 4);
-                else if (Pa == 2) NUDIM_GATHER(false, 2);
+                if (Pl == 8) NUDIM_GATHER(false, 8);
+                else if (Pl == 4) NUDIM_GATHER(false, 4);
+                else if (Pl == 2) NUDIM_GATHER(false, 2);
                 else NUDIM_GATHER(false, 1);
             }
 #undef NUDIM_GATHER
