@@ -204,6 +204,7 @@ template <typename T> struct NfftDev {
     int nE = 0;                     // trafo entries; their records (structure of arrays):
     int *e_rb = nullptr, *e_cc = nullptr;
     T *e_qa = nullptr, *e_q1 = nullptr;
+    int Ew = 0;  // FP64: e_qa and band_w as fixed point under this exponent field (0: as FP64)
     unsigned char *nslots = nullptr;
 
     // uploads go on stream st (tables are consumed by later work on st)

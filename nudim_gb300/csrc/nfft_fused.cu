@@ -24,6 +24,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "fixed.cuh"
 #include "engine.cuh"
 #include "fft_regs.cuh"
 
@@ -117,6 +118,88 @@ __device__ cplx_t<T> *block_fft(cplx_t<T> *a, cplx_t<T> *b, int n, int logn, int
 }
 
 
+// ================================================================ FP64 sums in integers
+static int exp_field(double x)  // of a positive normal x
+{
+    int e;
+    std::frexp(x, &e);
+    return e + 1022;
+}
+
+// weights to fixed point in place
+__global__ void __launch_bounds__(256) k_fix_weights(double *w, size_t n, int Ew)
+{
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    if (i < n) *reinterpret_cast<Fixed *>(w + i) = to_fixed(w[i], Ew);
+}
+
+// The column block's values (cnt of them) to fixed point in place (all threads).
+// Returns their exponent field, or -1 where they stay FP64.
+__device__ __forceinline__ int fix_columns(double2 *G, int cnt, int Ew, int *sh)
+{
+    int E = 0;
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+        E = max(E, max(exp_of(G[i].x), exp_of(G[i].y)));
+    E = __reduce_max_sync(0xffffffffu, E);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = E;
+    __syncthreads();
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) E = max(E, sh[w]);
+    if (!Ew || !fixed_range(E)) return -1;
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+        const FixedC v{to_fixed(G[i].x, E), to_fixed(G[i].y, E)};
+        *reinterpret_cast<FixedC *>(G + i) = v;
+    }
+    __syncthreads();
+    return E;
+}
+
+// A node's window over the block's columns in the FP64 form: row weights as
+// fixed point (exponent field Ew), column q of the entry at gp(q). The rows are
+// summed in integers, the columns in FP64 (those in integers too: as long, and an
+// error up to twice as large).
+template <typename F>
+__device__ __forceinline__ double2 window_fp64(const double *__restrict__ qa,
+                                               const double *__restrict__ q1, size_t nE, int e,
+                                               int odd, int rb, int m0, int cnt, int Ew, int Ev,
+                                               F gp)
+{
+    // the window's 14 rows (the 16 weights start at the even row below)
+    qa += odd * nE + e;
+    double ar = 0, ai = 0;
+    if (Ev >= 0) {
+        Fixed w[14];
+#pragma unroll
+        for (int i = 0; i < 14; i++) w[i] = *reinterpret_cast<const Fixed *>(qa + i * nE);
+        for (int q = 0; q < cnt; q++) {
+            const FixedC *g = reinterpret_cast<const FixedC *>(gp(q));
+            FixedSum s;
+            s.init();
+#pragma unroll
+            for (int i = 0; i < 14; i++) s.add(w[i], g[(rb + odd + i) & m0]);
+            const double w1 = q1[(size_t)q * nE + e];
+            ar = fma(w1, s.re(), ar);
+            ai = fma(w1, s.im(), ai);
+        }
+        const double sc = fixed_scale(Ew, Ev);
+        return make_double2(ar * sc, ai * sc);
+    }
+    for (int q = 0; q < cnt; q++) {
+        const double2 *g = gp(q);
+        double sr = 0, si = 0;
+#pragma unroll
+        for (int i = 0; i < 14; i++) {
+            const double wv = fixed_value(qa + i * nE, Ew);
+            const double2 v = g[(rb + odd + i) & m0];
+            sr = fma(wv, v.x, sr);
+            si = fma(wv, v.y, si);
+        }
+        const double w1 = q1[(size_t)q * nE + e];
+        ar = fma(w1, sr, ar);
+        ai = fma(w1, si, ai);
+    }
+    return make_double2(ar, ai);
+}
+
 // ================================================================ K1 row pass (trafo)
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
@@ -198,7 +281,7 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
                 const int *__restrict__ ent, const int *__restrict__ e_rb,
                 const int *__restrict__ e_cc, const T *__restrict__ e_qa,
                 const T *__restrict__ e_q1, int nE, int M, int smax,
-                cplx_t<T> *__restrict__ part)
+                cplx_t<T> *__restrict__ part, int Ew)
 {
     using C = cplx_t<T>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -231,21 +314,30 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
         }
     }
     __syncthreads();
-    const C *G = block_fft<T, -1>(A, B, n0, logn0, BC, tw0);
+    C *G = block_fft<T, -1>(A, B, n0, logn0, BC, tw0);
+    int Ev = 0;
+    if constexpr (sizeof(T) == 8) {
+        __shared__ int she[32];
+        Ev = fix_columns(G, BC * n0, Ew, she);
+    }
     const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
         const int cl0 = ccn & 255, cnt = (ccn >> 8) & 255;
-        T qa[16];
+        if constexpr (sizeof(T) == 8) {
+            part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] =
+                window_fp64(e_qa, e_q1, nE, e, ccn >> 16, rb, m0, cnt, Ew, Ev, [&](int q) {
+                    return G + (size_t)((cl0 + q) & (BC - 1)) * n0;
+                });
+        } else {
+            T qa[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) qa[i] = e_qa[(size_t)i * nE + e];
-        T ar = 0, ai = 0;
-        for (int q = 0; q < cnt; q++) {
-            const C *gp = G + (size_t)((cl0 + q) & (BC - 1)) * n0;
-            T sr = 0, si = 0;
-            if constexpr (sizeof(T) == 4) {
-                // FP32 form: one paired FMA per row, (re, im) += q * g
+            for (int i = 0; i < 16; i++) qa[i] = e_qa[(size_t)i * nE + e];
+            T ar = 0, ai = 0;
+            for (int q = 0; q < cnt; q++) {
+                const C *gp = G + (size_t)((cl0 + q) & (BC - 1)) * n0;
+                // one paired FMA per row, (re, im) += q * g
                 float2 s2 = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
@@ -254,25 +346,12 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
                     s2 = __ffma2_rn(make_float2(qa[2 * i + 1], qa[2 * i + 1]),
                                     make_float2(pr.z, pr.w), s2);
                 }
-                sr = s2.x;
-                si = s2.y;
-            } else {
-                // FP64: the window's 14 rows only (the 16-row pairs are an
-                // FP32 load shape; every FMA counts on the FP64 pipe)
-                const int odd = ccn >> 16;
-#pragma unroll
-                for (int i = 0; i < 14; i++) {
-                    const T w = odd ? qa[i + 1] : qa[i];
-                    C g = gp[(rb + odd + i) & m0];
-                    sr += w * g.x;
-                    si += w * g.y;
-                }
+                T w = e_q1[(size_t)q * nE + e];
+                ar += w * s2.x;
+                ai += w * s2.y;
             }
-            T w = e_q1[(size_t)q * nE + e];
-            ar += w * sr;
-            ai += w * si;
+            part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] = mkc<T>(ar, ai);
         }
-        part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] = mkc<T>(ar, ai);
     }
 }
 
@@ -282,17 +361,21 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
 // of H straight into pass 1's registers (a warp reads 8 rows x 4 columns
 // per step), exchange through shared memory, and pass 2 writes the columns
 // to Gs (column stride n0 + 8: the four columns' stores meet distinct
-// banks); then every thread interpolates as in k_colfft_interp.
-template <typename T, int R1, int R2>
-__global__ void __launch_bounds__(32 * col_warps<T>(), sizeof(T) == 4 ? NUDIM_COL_MINB : 1)
-k_colfft_interp_fs(const cplx_t<T> *__restrict__ H, int N0, int n1,
-                   const cplx_t<T> *__restrict__ tw0, const int4 *__restrict__ units,
+// banks); then every thread interpolates as in k_colfft_interp. FP64 (the FP32
+// form has the kernels below). The FP64 unit's FFTs and the integer sums of
+// other CTAs overlap: two CTAs an SM where the registers allow (n0 = 256; 24
+// planes at 128^2: 344 -> 235 us).
+template <int R1, int R2>
+__global__ void __launch_bounds__(32 * col_warps<double>(), R1 == 16 ? 2 : 1)
+k_colfft_interp_fs(const double2 *__restrict__ H, int N0, int n1,
+                   const double2 *__restrict__ tw0, const int4 *__restrict__ units,
                    const int *__restrict__ ent, const int *__restrict__ e_rb,
-                   const int *__restrict__ e_cc, const T *__restrict__ e_qa,
-                   const T *__restrict__ e_q1, int nE, int M, int smax,
-                   cplx_t<T> *__restrict__ part)
+                   const int *__restrict__ e_cc, const double *__restrict__ e_qa,
+                   const double *__restrict__ e_q1, int nE, int M, int smax,
+                   double2 *__restrict__ part, int Ew)
 {
-    using C = cplx_t<T>;
+    using T = double;
+    using C = double2;
     constexpr int n0 = R1 * R2, BC = 4, GS = n0 + 8, CS = fs_col_stride<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
     C *Gs = (C *)smraw, *S = Gs + BC * GS;
@@ -329,47 +412,20 @@ k_colfft_interp_fs(const cplx_t<T> *__restrict__ H, int N0, int n1,
             for (int k2 = 0; k2 < R2; k2++) Gs[c * GS + k1 + R1 * k2] = y[fs_out<R2>(k2)];
         }
     }
+    // (the columns' padding, which fix_columns passes over)
+    for (int i = threadIdx.x; i < BC * (GS - n0); i += blockDim.x)
+        Gs[(i / (GS - n0)) * GS + n0 + i % (GS - n0)] = mkc<T>(0, 0);
     __syncthreads();
+    __shared__ int she[32];
+    const int Ev = fix_columns(Gs, BC * GS, Ew, she);
     const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
         const int cl0 = ccn & 255, cnt = (ccn >> 8) & 255;
-        T qa[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) qa[i] = e_qa[(size_t)i * nE + e];
-        T ar = 0, ai = 0;
-        for (int q = 0; q < cnt; q++) {
-            const C *gp = Gs + (size_t)((cl0 + q) & (BC - 1)) * GS;
-            T sr = 0, si = 0;
-            if constexpr (sizeof(T) == 4) {
-                float2 s2 = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    float4 pr = *(const float4 *)(gp + ((rb + 2 * i) & m0));
-                    s2 = __ffma2_rn(make_float2(qa[2 * i], qa[2 * i]), make_float2(pr.x, pr.y), s2);
-                    s2 = __ffma2_rn(make_float2(qa[2 * i + 1], qa[2 * i + 1]),
-                                    make_float2(pr.z, pr.w), s2);
-                }
-                sr = s2.x;
-                si = s2.y;
-            } else {
-                // FP64: the window's 14 rows only (the 16-row pairs are an
-                // FP32 load shape; every FMA counts on the FP64 pipe)
-                const int odd = ccn >> 16;
-#pragma unroll
-                for (int i = 0; i < 14; i++) {
-                    const T w = odd ? qa[i + 1] : qa[i];
-                    C g = gp[(rb + odd + i) & m0];
-                    sr += w * g.x;
-                    si += w * g.y;
-                }
-            }
-            T w = e_q1[(size_t)q * nE + e];
-            ar += w * sr;
-            ai += w * si;
-        }
-        part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] = mkc<T>(ar, ai);
+        part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] =
+            window_fp64(e_qa, e_q1, nE, e, ccn >> 16, rb, m0, cnt, Ew, Ev,
+                        [&](int q) { return Gs + (size_t)((cl0 + q) & (BC - 1)) * GS; });
     }
 }
 
@@ -703,7 +759,8 @@ constexpr int kGatherMaxEntries = 128;
 template <int P> __host__ __device__ constexpr int gather_fs_stride() { return P == 1 ? 1 : P + 2; }
 template <typename T, int P> __host__ __device__ constexpr size_t gather_stage_bytes(int W)
 {
-    return 32 * ((size_t)W * sizeof(T) + (size_t)gather_fs_stride<P>() * sizeof(cplx_t<T>));
+    const size_t b = 32 * ((size_t)W * sizeof(T) + (size_t)gather_fs_stride<P>() * sizeof(cplx_t<T>));
+    return sizeof(T) == 8 ? b + P * 32 * sizeof(double2) + 32 : b;
 }
 
 // The units of a CTA for its group's np <= P planes from pb on.
@@ -711,7 +768,7 @@ template <typename T, bool WEIGHTED, int P>
 __device__ __forceinline__ void
 gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, int t1, int &next_tile,
              const int *__restrict__ band_node, const T *__restrict__ band_w, int nbands, int n0,
-             int n1, int BC, int nb_planes, int plane0, int pb, int np, unsigned char *smraw,
+             int n1, int BC, int nb_planes, int plane0, int pb, int np, int Ew, unsigned char *smraw,
              cplx_t<T> *__restrict__ G, cplx_t<T> *__restrict__ part)
 {
     using C = cplx_t<T>;
@@ -720,6 +777,10 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
     const int R = 32 / BC, W = R + BC;
     T *ws = (T *)(smraw + warp * gather_stage_bytes<T, P>(W));  // [32][W] weights
     C *fs = (C *)(ws + 32 * W);                                 // [32][FS] node values
+    // FP64: the totals [P][32] and the chunk's exponents [P]; the integer sums
+    // take the registers
+    C *tot = fs + 32 * FS;
+    int *es = (int *)(tot + P * 32);
     const int rr = lane / BC, cc = lane - rr * BC;
     const int wv16 = W * (int)sizeof(T) / 16;  // 16-byte vectors of an entry's weights
     const C *f0 = sa.f + (size_t)(plane0 + pb) * sa.f_stride;
@@ -728,15 +789,17 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
     while (it < t1) {
         const int4 un = units[it];  // tile, first entry, end, partial slot (0: G)
         const int tile = un.x, beg = un.y, end = un.z;
-        T ar[P], ai[P];
         Kahan2 ks[P];  // FP32: compensated totals of the chunk sums (re, im)
 #pragma unroll
         for (int p = 0; p < P; p++) {
-            ar[p] = ai[p] = T(0);
+            if (sizeof(T) == 8) tot[p * 32 + lane] = mkc<T>(0, 0);
             ks[p].init();
         }
         for (int base = beg; base < end; base += 32) {
             const int n = min(32, end - base);
+            C fv[P];
+#pragma unroll
+            for (int p = 0; p < P; p++) fv[p] = mkc<T>(0, 0);
             if (lane < n) {
                 const int e = base + lane;
                 const int j = band_node[e];
@@ -745,16 +808,38 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
                 for (int q = 0; q < wv16; q++) dst[q] = src[q];
                 const T wv = WEIGHTED ? sa.w[j] : T(1);
                 const C *fp = f0 + j;
-                C fv[P];
 #pragma unroll
                 for (int p = 0; p < P; p++) {
-                    fv[p] = mkc<T>(0, 0);
                     if (p < np) fv[p] = *fp;
                     fp += sa.f_stride;
                 }
+                if (WEIGHTED)
 #pragma unroll
-                for (int p = 0; p < P; p++)
-                    fs[lane * FS + p] = WEIGHTED ? mkc<T>(wv * fv[p].x, wv * fv[p].y) : fv[p];
+                    for (int p = 0; p < P; p++) fv[p] = mkc<T>(wv * fv[p].x, wv * fv[p].y);
+                if (sizeof(T) == 4)
+#pragma unroll
+                    for (int p = 0; p < P; p++) fs[lane * FS + p] = fv[p];
+            }
+            bool ints = Ew > 0;
+            if constexpr (sizeof(T) == 8) {
+                // FP64: each plane's values under the chunk's largest exponent
+                int E[P];
+#pragma unroll
+                for (int p = 0; p < P; p++) {
+                    E[p] = __reduce_max_sync(0xffffffffu, max(exp_of(fv[p].x), exp_of(fv[p].y)));
+                    ints = ints && fixed_range(E[p]);
+                    if (lane == p) es[p] = E[p];
+                }
+                if (lane < n)
+#pragma unroll
+                    for (int p = 0; p < P; p++) {
+                        if (ints) {
+                            const FixedC v{to_fixed(fv[p].x, E[p]), to_fixed(fv[p].y, E[p])};
+                            *reinterpret_cast<FixedC *>(fs + lane * FS + p) = v;
+                        } else {
+                            fs[lane * FS + p] = fv[p];
+                        }
+                    }
             }
             __syncwarp();
             if constexpr (sizeof(T) == 4) {
@@ -789,16 +874,37 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
                     for (int p = 0; p < P; p++) ks[p].add(bs[p]);
                 }
             } else {
-                // FP64: the point's weight once per entry, then one fused
-                // multiply-add per plane and component (the FP64 pipe is
-                // the bound on this GPU)
-                for (int k = 0; k < n; k++) {
-                    const T q = ws[k * W + rr] * ws[k * W + R + cc];
+                // FP64: the point's weight once per entry, the chunk's sums in
+                // integers (one fused multiply-add per plane and component
+                // where the values' range does not allow it)
+                if (ints) {
+                    FixedSum a[P];
+#pragma unroll
+                    for (int p = 0; p < P; p++) a[p].init();
+#pragma unroll 1
+                    for (int k = 0; k < n; k++) {
+                        const Fixed *wk = reinterpret_cast<const Fixed *>(ws + k * W);
+                        const Fixed q = fixed_product(wk[rr], wk[R + cc]);
+#pragma unroll
+                        for (int p = 0; p < P; p++)
+                            a[p].add(q, *reinterpret_cast<const FixedC *>(fs + k * FS + p));
+                    }
 #pragma unroll
                     for (int p = 0; p < P; p++) {
-                        const C fv = fs[k * FS + p];
-                        ar[p] = fma(q, fv.x, ar[p]);
-                        ai[p] = fma(q, fv.y, ai[p]);
+                        const double sc = fixed_scale(2 * Ew - 1022, es[p]);
+                        C &t = tot[p * 32 + lane];
+                        t = mkc<T>(fma(a[p].re(), sc, t.x), fma(a[p].im(), sc, t.y));
+                    }
+                } else {
+                    for (int k = 0; k < n; k++) {
+                        const T q = fixed_value(ws + k * W + rr, Ew) *
+                                    fixed_value(ws + k * W + R + cc, Ew);
+#pragma unroll
+                        for (int p = 0; p < P; p++) {
+                            const C v = fs[k * FS + p];
+                            C &t = tot[p * 32 + lane];
+                            t = mkc<T>(fma(q, v.x, t.x), fma(q, v.y, t.y));
+                        }
                     }
                 }
             }
@@ -810,12 +916,10 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
         const size_t step = un.w == 0 ? (size_t)n0 * n1 : 32;
 #pragma unroll
         for (int p = 0; p < P; p++) {
-            if (sizeof(T) == 4) {
-                const float2 v = ks[p].value();
-                ar[p] = (T)v.x;
-                ai[p] = (T)v.y;
-            }
-            if (p < np) *out = mkc<T>(ar[p], ai[p]);
+            C v;
+            if constexpr (sizeof(T) == 4) v = ks[p].value();
+            else v = tot[p * 32 + lane];
+            if (p < np) *out = v;
             out += step;
         }
         int nt = 0;
@@ -824,13 +928,16 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
     }
 }
 
-// A last group of at most half the planes takes the loop for so many.
+// A last group of at most half the planes takes the loop for so many. FP64: the
+// integer sums of 8 planes are 64 registers, so two CTAs an SM, with the totals in
+// shared memory (in registers they spill: 336 us against 261 for 24 planes at
+// 128^2; 4 planes at a time 268; FP64 sums 781).
 template <typename T, bool WEIGHTED, int P>
-__global__ void __launch_bounds__(32 * kGatherWarps, 3)
+__global__ void __launch_bounds__(32 * kGatherWarps, sizeof(T) == 4 ? 3 : 2)
 k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits, int upc,
                 const int *__restrict__ band_node, const T *__restrict__ band_w, int nbands,
                 int n0, int n1, int BC, int nb_planes, int plane0, cplx_t<T> *__restrict__ G,
-                cplx_t<T> *__restrict__ part)
+                cplx_t<T> *__restrict__ part, int Ew)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int next_tile;
@@ -841,7 +948,7 @@ k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits, in
     __syncthreads();
 #define NUDIM_UNITS(PP)                                                                          \
     gather_units<T, WEIGHTED, PP>(sa, units, t0, t1, next_tile, band_node, band_w, nbands, n0,   \
-                                  n1, BC, nb_planes, plane0, pb, np, smraw, G, part)
+                                  n1, BC, nb_planes, plane0, pb, np, Ew, smraw, G, part)
     if constexpr (P >= 8) {
         if (np <= 2) NUDIM_UNITS(2);
         else if (np <= 4) NUDIM_UNITS(4);
@@ -1271,7 +1378,7 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
     smem_colifft = 2 * sizeof(C) * fft_buf((size_t)BCa * n0);
     // The limit is a property of the kernel, shared by every plan in the
     // process: set it to the largest size any plan uses (never lower it).
-    const int lim_col = 144 << 10, lim_row = 112 << 10, lim_spread = 96 << 10,
+    const int lim_col = 144 << 10, lim_row = 112 << 10, lim_spread = 112 << 10,
               lim_colifft = 144 << 10;
     if (rows < 1 || smem_col > (size_t)lim_col || smem_row > (size_t)lim_row ||
         smem_spread > (size_t)lim_spread || smem_colifft > (size_t)lim_colifft) {
@@ -1320,6 +1427,21 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
     NUDIM_TRY(up((void **)&units, hu.data(), sizeof(int4) * hu.size()));
     if (!hf.empty()) NUDIM_TRY(up((void **)&fixups, hf.data(), sizeof(int4) * hf.size()));
     NUDIM_TRY(up((void **)&band_w, L.band_w.data(), sizeof(T) * L.band_w.size()));
+    if constexpr (sizeof(T) == 8) {
+        // the row weights and the tiles' weights as fixed point under the largest
+        // one's exponent, unless one is no number
+        double m = 0;
+        bool finite = true;
+        for (const double v : t.psi) {
+            finite = finite && std::isfinite(v);
+            m = std::max(m, std::fabs(v));
+        }
+        Ew = finite && m > 1e-30 && m < 1e30 ? exp_field(m) : 0;
+        const size_t na = L.ent_qa.size(), nw = L.band_w.size();
+        if (Ew && na) k_fix_weights<<<ceil_div(na, 256), 256, 0, st>>>(e_qa, na, Ew);
+        if (Ew && nw) k_fix_weights<<<ceil_div(nw, 256), 256, 0, st>>>(band_w, nw, Ew);
+        NUDIM_LAUNCH_CHECK();
+    }
     NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     lim_col));
     {
@@ -1370,11 +1492,11 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, lim_col));
     NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs2<16, 16>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, lim_col));
-    NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<T, 32, 32>,
+    NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<32, 32>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, lim_col));
-    NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<T, 32, 16>,
+    NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<32, 16>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, lim_col));
-    NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<T, 16, 16>,
+    NUDIM_CUDA(cudaFuncSetAttribute(k_colfft_interp_fs<16, 16>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, lim_col));
     // the four-step column IFFTs' exchange buffers (FP64 1024 points: 68 KB)
     NUDIM_CUDA(cudaFuncSetAttribute(k_colifft_fs<T, 32, 32>,
@@ -1486,8 +1608,9 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             // one radix-16 butterfly per thread: 64 threads per column
             const int thr = std::min(32 * col_warps<T>(), std::max(64, 64 * BC));
 #define NUDIM_COLFS(R1, R2)                                                                      \
-    k_colfft_interp_fs<T, R1, R2><<<dim3(nc, nb), thr, smem_colfs_of<T>(R1, R2), st>>>(             \
-        H, N0, n1, tw0, cu, ent, e_rb, e_cc, e_qa, e_q1, nE, M, smax, P)
+    k_colfft_interp_fs<R1, R2><<<dim3(nc, nb), thr, smem_colfs_of<double>(R1, R2), st>>>(           \
+        (const double2 *)H, N0, n1, (const double2 *)tw0, cu, ent, e_rb, e_cc,                 \
+        (const double *)e_qa, (const double *)e_q1, nE, M, smax, (double2 *)P, Ew)
 #define NUDIM_COLFS2(R1, R2)                                                                     \
     k_colfft_interp_fs2<R1, R2><<<dim3(nc, ceil_div(nb, 2)), 256,                             \
                                   sizeof(float2) * 2 * 4 * fs2_gs<R1, R2>(), st>>>(             \
@@ -1510,7 +1633,7 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             else
                 k_colfft_interp<T><<<dim3(nc, nb), thr, smem_col, st>>>(
                     H, N0, n0, logn0, n1, BC, tw0, cu, ent, e_rb, e_cc, e_qa, e_q1, nE, M,
-                    smax, P);
+                    smax, P, Ew);
 #undef NUDIM_COLFS
 #undef NUDIM_COLFS2
 #undef NUDIM_COLFS8
@@ -1563,7 +1686,7 @@ int NfftDev<T>::adjoint_fused(int nplanes, const SpreadArgs<T> &sa, const CropAr
 #define NUDIM_GATHER(WT, PP)                                                                    \
     k_spread_gather<T, WT, PP><<<g, thr, smem_spread, st>>>(sa, units, nunits, upc, band_node,  \
                                                             band_w, nbands, n0, n1, BCa, nb,    \
-                                                            p0, G, part)
+                                                            p0, G, part, Ew)
             if (sa.w) {
                 if (Pl == 8) NUDIM_GATHER(true, 8);
                 else if (Pl == 4) NUDIM_GATHER(true, 4);
