@@ -208,17 +208,17 @@ __device__ __forceinline__ double tv_root(double s)
 // r < kTvRows.  done: a zeroed counter (the last block resets it).
 //
 // FUSED: the previous iteration's update is applied as the tile is read
-// (u' = u - step_in[1] (g_in / step_in[0]) on every tile and halo cell, with k_tv_update's operations), the owned cells' u' are
-// written to u_out and the gradient of u' to g: one pass reads u and g_in and
+// (u' = u - step_in[1] (g_in / step_in[0]) on every tile and halo cell, with
+// k_tv_update's operations), the owned cells' u' are written to u_out and the gradient of u' to g: one pass reads u and g_in and
 // writes u' and g (4 values per voxel instead of the 5 of a gradient and an
 // update).  u_out and g must not alias u and g_in (other blocks still read
 // their halos).
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(256, kTvSumBlocks<T>)
-k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
-          unsigned *__restrict__ done, double *__restrict__ step, int nz, int ny, int nx,
-          int zc, int runs, int rep, int height, int ylo, int yhi, const T *__restrict__ g_in,
-          const double *__restrict__ step_in, double lam, T *__restrict__ u_out)
+k_tv_grad(const T *u, T *g, double *part,
+          unsigned *done, double *step, int nz, int ny, int nx,
+          int zc, int runs, int rep, int height, int ylo, int yhi, const T *g_in,
+          const double *step_in, double lam, T *u_out)
 {
     constexpr int kCells = kTvSY * kTvSX, kSlots = (kCells + 255) / 256;
     constexpr bool FLOAT = sizeof(T) == 4;
@@ -279,8 +279,7 @@ k_tv_grad(const T *__restrict__ u, T *__restrict__ g, double *__restrict__ part,
         }
         __pipeline_commit();
     };
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    await_last();
     TvNorm<T> norm;
     // u' in slot `sl`: each thread its own cells, so its own copies' arrival is
     // all it waits for
@@ -480,11 +479,10 @@ template <typename T, int N> struct alignas(sizeof(T) * N) TvVec {
 // same values).
 template <typename T, typename I, int VEC>
 __global__ void __launch_bounds__(256)
-k_tv_update(const T *u, T *u_out, const T *__restrict__ g, const double *__restrict__ step,
+k_tv_update(const T *u, T *u_out, const T *g, const double *step,
             int nz, int ny, int nx, int height, int ylo, int yhi)
 {
-    cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
+    await_last();
     TvNorm<T> tn;
     tn.init((T)step[0]);
     const T la = (T)step[1];
@@ -521,24 +519,6 @@ template <typename T> static bool tv_unfused()
     if (e && !strcmp(e, "unfused")) return true;
     if (e && !strcmp(e, "fused")) return false;
     return sizeof(T) == 8;
-}
-
-// A launch that starts while the one before it still runs and waits for its end
-// before the first access (a chain of small volumes' passes is bound by latency:
-// 16 x 48 x 40, 40 steps, 500 -> 404 us).
-template <typename... P, typename... A>
-static cudaError_t launch_early(void (*kern)(P...), dim3 grid, cudaStream_t st, A... args)
-{
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c{};
-    c.gridDim = grid;
-    c.blockDim = dim3(256);
-    c.stream = st;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
 }
 
 template <typename T, typename I>
@@ -582,11 +562,11 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     // the pointers' alignment
     auto update = [&](const T *uin, T *uout, const T *gv, const double *sc) -> int {
         if (wide(uin, uout, gv))
-            NUDIM_CUDA(launch_early(k_tv_update<T, I, W>, dim3((unsigned)nuw), st, uin, uout, gv,
-                                    sc, nz, ny, nx, height, ylo, yhi));
+            launch_early(k_tv_update<T, I, W>, (int)nuw, 256, 0, st, uin, uout, gv, sc, nz, ny, nx,
+                         height, ylo, yhi);
         else
-            NUDIM_CUDA(launch_early(k_tv_update<T, I, 1>, dim3((unsigned)nu1), st, uin, uout, gv,
-                                    sc, nz, ny, nx, height, ylo, yhi));
+            launch_early(k_tv_update<T, I, 1>, (int)nu1, 256, 0, st, uin, uout, gv, sc, nz, ny, nx,
+                         height, ylo, yhi);
         NUDIM_LAUNCH_CHECK();
         return NUDIM_OK;
     };
@@ -613,8 +593,8 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     for (int it = 1; it < niter; it++) {
         T *nu = cu == u ? u2 : u, *ng = cg == grad ? g2 : grad;
         double *ns = cs == scal ? scal + 2 : scal;
-        NUDIM_CUDA(launch_early(k_tv_grad<T, true>, gg, st, cu, ng, part, done, ns, nz, ny, nx, zc,
-                                runs, rep, height, ylo, yhi, cg, cs, (double)lam, nu));
+        launch_early(k_tv_grad<T, true>, gg, 256, 0, st, cu, ng, part, done, ns, nz, ny, nx, zc,
+                     runs, rep, height, ylo, yhi, cg, cs, (double)lam, nu);
         NUDIM_LAUNCH_CHECK();
         cu = nu;
         cg = ng;

@@ -174,9 +174,10 @@ template <> int fft_exec<float>(cufftHandle h, float2 *io, int dir)
 }
 
 // ================================================================ reductions
-__global__ void k_finish_sums(const double *__restrict__ part, int nparts, int stride_in,
-                              double *__restrict__ out, int out_stride)
+__global__ void k_finish_sums(const double *part, int nparts, int stride_in,
+                              double *out, int out_stride)
 {
+    await_last();
     __shared__ double sh[32];
     int b = blockIdx.x, k = blockIdx.y;
     const double *src = part + (size_t)b * stride_in + (size_t)k * nparts;
@@ -189,8 +190,8 @@ __global__ void k_finish_sums(const double *__restrict__ part, int nparts, int s
 void launch_finish_sums(const double *part, int nparts, int nplanes, int stride_in,
                         double *out, int out_stride, int nsums, cudaStream_t st)
 {
-    k_finish_sums<<<dim3(nplanes, nsums), 256, 0, st>>>(part, nparts, stride_in, out,
-                                                         out_stride);
+    launch_early(k_finish_sums, dim3(nplanes, nsums), 256, 0, st, part, nparts, stride_in, out,
+                 out_stride);
     ++g_launches;
 }
 

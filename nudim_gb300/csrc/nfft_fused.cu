@@ -203,11 +203,12 @@ __device__ __forceinline__ double2 window_fp64(const double *__restrict__ qa,
 // ================================================================ K1 row pass (trafo)
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
-k_rowfft(const void *__restrict__ src, size_t src_stride, int N0, int N1, int n1, int logn1,
+k_rowfft(const void *src, size_t src_stride, int N0, int N1, int n1, int logn1,
          int kRows, const T *__restrict__ c0, const T *__restrict__ c1,
-         const cplx_t<T> *__restrict__ tw1, int plane0, cplx_t<T> *__restrict__ H,
-         cplx_t<T> *__restrict__ f_init, size_t f_stride)
+         const cplx_t<T> *__restrict__ tw1, int plane0, cplx_t<T> *H,
+         cplx_t<T> *f_init, size_t f_stride)
 {
+    await_last();
     using C = cplx_t<T>;
     extern __shared__ __align__(16) unsigned char smraw[];
     C *A = (C *)smraw, *B = A + fft_buf((size_t)kRows * n1);
@@ -276,13 +277,14 @@ template <typename T> __host__ __device__ constexpr int col_warps() { return 8; 
 #endif
 template <typename T>
 __global__ void __launch_bounds__(32 * col_warps<T>(), sizeof(T) == 4 ? NUDIM_COL_MINB : 1)
-k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int n1, int BC,
+k_colfft_interp(const cplx_t<T> *H, int N0, int n0, int logn0, int n1, int BC,
                 const cplx_t<T> *__restrict__ tw0, const int4 *__restrict__ units,
                 const int *__restrict__ ent, const int *__restrict__ e_rb,
                 const int *__restrict__ e_cc, const T *__restrict__ e_qa,
                 const T *__restrict__ e_q1, int nE, int M, int smax,
-                cplx_t<T> *__restrict__ part, int Ew)
+                cplx_t<T> *part, int Ew)
 {
+    await_last();
     using C = cplx_t<T>;
     extern __shared__ __align__(16) unsigned char smraw[];
     C *A = (C *)smraw, *B = A + fft_buf((size_t)BC * n0);
@@ -367,13 +369,14 @@ k_colfft_interp(const cplx_t<T> *__restrict__ H, int N0, int n0, int logn0, int 
 // planes at 128^2: 344 -> 235 us).
 template <int R1, int R2>
 __global__ void __launch_bounds__(32 * col_warps<double>(), R1 == 16 ? 2 : 1)
-k_colfft_interp_fs(const double2 *__restrict__ H, int N0, int n1,
+k_colfft_interp_fs(const double2 *H, int N0, int n1,
                    const double2 *__restrict__ tw0, const int4 *__restrict__ units,
                    const int *__restrict__ ent, const int *__restrict__ e_rb,
                    const int *__restrict__ e_cc, const double *__restrict__ e_qa,
                    const double *__restrict__ e_q1, int nE, int M, int smax,
-                   double2 *__restrict__ part, int Ew)
+                   double2 *part, int Ew)
 {
+    await_last();
     using T = double;
     using C = double2;
     constexpr int n0 = R1 * R2, BC = 4, GS = n0 + 8, CS = fs_col_stride<R1, R2>();
@@ -447,13 +450,14 @@ template <int R1, int R2> __host__ __device__ constexpr int fs2_gs()
 
 template <int R1, int R2>
 __global__ void __launch_bounds__(256, 3)
-k_colfft_interp_fs2(const float2 *__restrict__ H, int N0, int n1, int nb_planes,
+k_colfft_interp_fs2(const float2 *H, int N0, int n1, int nb_planes,
                     const float2 *__restrict__ tw0, const int4 *__restrict__ units,
                     const int *__restrict__ ent, const int *__restrict__ e_rb,
                     const int *__restrict__ e_cc, const float *__restrict__ e_qa,
                     const float *__restrict__ e_q1, int nE, int M, int smax,
-                    float2 *__restrict__ part)
+                    float2 *part)
 {
+    await_last();
     using C = float2;
     constexpr int n0 = R1 * R2, BC = 4, GS = fs2_gs<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -560,13 +564,14 @@ template <int R1, int R2> __host__ __device__ constexpr int fs8_gs()
 
 template <int R1, int R2>
 __global__ void __launch_bounds__(256, 3)
-k_colfft_interp_fs8(const float2 *__restrict__ H, int N0, int n1,
+k_colfft_interp_fs8(const float2 *H, int N0, int n1,
                     const float2 *__restrict__ tw0, const int4 *__restrict__ units,
                     const int *__restrict__ ent, const int *__restrict__ e_rb,
                     const int *__restrict__ e_cc, const float *__restrict__ e_qa,
                     const float *__restrict__ e_q1, int nE, int M, int smax,
-                    float2 *__restrict__ part)
+                    float2 *part)
 {
+    await_last();
     using C = float2;
     constexpr int n0 = R1 * R2, BC = 8, GS = fs8_gs<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -644,9 +649,10 @@ k_colfft_interp_fs8(const float2 *__restrict__ H, int N0, int n1,
 // ================================================================ K3 combine + epilogue
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
-k_combine(const cplx_t<T> *__restrict__ part, const unsigned char *__restrict__ nslots, int M,
+k_combine(const cplx_t<T> *part, const unsigned char *__restrict__ nslots, int M,
           int smax, int plane0, InterpArgs<T> a)
 {
+    await_last();
     using C = cplx_t<T>;
     __shared__ double sh[32];
     int b = blockIdx.y, gb = plane0 + b;
@@ -736,8 +742,8 @@ struct Kahan2 {
 // shared-memory stage, then every lane sums, for its grid point and each
 // plane, q0(row) q1(col) f over the chunk -- one paired FMA per plane and
 // entry in FP32.  FP32: plain sums within a chunk, Kahan-compensated across
-// chunks; FP64: fused multiply-adds in ascending node order.  The tile's 32 points of each plane are one
-// contiguous 256-byte (FP32) store: G is laid out column block by column
+// chunks; FP64: a chunk's sum in integers (fixed.cuh), the chunks in order.  The
+// tile's 32 points of each plane are one contiguous 256-byte (FP32) store: G is laid out column block by column
 // block, [plane][block][row][column in block], which is also the order the
 // column IFFT reads.  The work units are ranges of at most kGatherMaxEntries
 // entries of a tile's list (the lists near the polar grid's centre run to
@@ -935,10 +941,11 @@ gather_units(const SpreadArgs<T> &sa, const int4 *__restrict__ units, int t0, in
 template <typename T, bool WEIGHTED, int P>
 __global__ void __launch_bounds__(32 * kGatherWarps, sizeof(T) == 4 ? 3 : 2)
 k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits, int upc,
-                const int *__restrict__ band_node, const T *__restrict__ band_w, int nbands,
-                int n0, int n1, int BC, int nb_planes, int plane0, cplx_t<T> *__restrict__ G,
-                cplx_t<T> *__restrict__ part, int Ew)
+                const int *__restrict__ band_node, const T *band_w, int nbands,
+                int n0, int n1, int BC, int nb_planes, int plane0, cplx_t<T> *G,
+                cplx_t<T> *part, int Ew)
 {
+    await_last();
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int next_tile;
     const int pb = blockIdx.y * P, np = min(P, nb_planes - pb);
@@ -966,8 +973,9 @@ k_spread_gather(SpreadArgs<T> sa, const int4 *__restrict__ units, int nunits, in
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_spread_fixup(const int4 *__restrict__ fix, int nbands, int n0, int n1, int BC,
-               int nb_planes, const cplx_t<T> *__restrict__ part, cplx_t<T> *__restrict__ G)
+               int nb_planes, const cplx_t<T> *part, cplx_t<T> *G)
 {
+    await_last();
     using C = cplx_t<T>;
     const int4 fx = fix[blockIdx.x];
     const int lane = threadIdx.x & 31, R = 32 / BC, nblk = n1 / BC;
@@ -1001,10 +1009,11 @@ template <int R1, int R2> __host__ __device__ constexpr int fs_row_stride() { re
 
 template <typename T, int MODE, int R1, int R2>
 __global__ void __launch_bounds__(128)
-k_rowfft_fs(const void *__restrict__ src, size_t src_stride, int N0, int N1,
+k_rowfft_fs(const void *src, size_t src_stride, int N0, int N1,
             const T *__restrict__ c0, const T *__restrict__ c1, const cplx_t<T> *__restrict__ tw1,
-            int plane0, cplx_t<T> *__restrict__ H, cplx_t<T> *__restrict__ f_init, size_t f_stride)
+            int plane0, cplx_t<T> *H, cplx_t<T> *f_init, size_t f_stride)
 {
+    await_last();
     using C = cplx_t<T>;
     constexpr int n1 = R1 * R2, RPC = 128 / R2;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -1054,10 +1063,11 @@ k_rowfft_fs(const void *__restrict__ src, size_t src_stride, int N0, int N1,
 
 template <typename T, int MODE, int R1, int R2>
 __global__ void __launch_bounds__(128)
-k_rowifft_crop_fs(const cplx_t<T> *__restrict__ Hp, int N0, int N1, const T *__restrict__ c0,
+k_rowifft_crop_fs(const cplx_t<T> *Hp, int N0, int N1, const T *__restrict__ c0,
                   const T *__restrict__ c1, const cplx_t<T> *__restrict__ tw1, int plane0,
                   CropArgs<T> ca)
 {
+    await_last();
     using C = cplx_t<T>;
     constexpr int n1 = R1 * R2, RPC = 128 / R2;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -1132,9 +1142,10 @@ template <typename T> static size_t smem_colfs_of(int R1, int R2)
 
 template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(4 * R2)
-k_colifft_fs(const cplx_t<T> *__restrict__ G, int N0, int n1, const cplx_t<T> *__restrict__ tw0,
-             cplx_t<T> *__restrict__ Hp)
+k_colifft_fs(const cplx_t<T> *G, int N0, int n1, const cplx_t<T> *__restrict__ tw0,
+             cplx_t<T> *Hp)
 {
+    await_last();
     using C = cplx_t<T>;
     constexpr int n0 = R1 * R2, BC = 4, CS = fs_col_stride<R1, R2>();
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -1180,9 +1191,10 @@ k_colifft_fs(const cplx_t<T> *__restrict__ G, int N0, int n1, const cplx_t<T> *_
 // n0-point FFTs, the N0 kept rows (a - N0/2 mod n0) written to H'.
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_colifft(const cplx_t<T> *__restrict__ G, int N0, int n0, int logn0, int n1, int BC,
-          const cplx_t<T> *__restrict__ tw0, cplx_t<T> *__restrict__ Hp)
+k_colifft(const cplx_t<T> *G, int N0, int n0, int logn0, int n1, int BC,
+          const cplx_t<T> *__restrict__ tw0, cplx_t<T> *Hp)
 {
+    await_last();
     using C = cplx_t<T>;
     extern __shared__ __align__(16) unsigned char smraw[];
     C *A = (C *)smraw, *B = A + fft_buf((size_t)BC * n0);
@@ -1225,10 +1237,11 @@ k_colifft(const cplx_t<T> *__restrict__ G, int N0, int n0, int logn0, int n1, in
 // ================================================================ K5 row IFFT + crop
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
-k_rowifft_crop(const cplx_t<T> *__restrict__ Hp, int N0, int N1, int n1, int logn1, int kRows,
+k_rowifft_crop(const cplx_t<T> *Hp, int N0, int N1, int n1, int logn1, int kRows,
                const T *__restrict__ c0, const T *__restrict__ c1,
                const cplx_t<T> *__restrict__ tw1, int plane0, CropArgs<T> ca)
 {
+    await_last();
     using C = cplx_t<T>;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ double sh[32];
@@ -1575,8 +1588,8 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             ProfScope ps(ctx, PK_PAD, st, nb * c * ((double)N0 * N1 + (double)N0 * n1));
             dim3 g(ceil_div(N0, rows), nb);
 #define NUDIM_ROWFS(MD, R1, R2)                                                                  \
-    k_rowfft_fs<T, MD, R1, R2><<<g, 128, smem_row, st>>>(pa.src, pa.src_stride, N0, N1, c0, c1, \
-                                                          tw1, p0, H, pa.f_init, pa.f_stride)
+    launch_early(k_rowfft_fs<T, MD, R1, R2>, g, 128, smem_row, st, pa.src, pa.src_stride, N0, \
+        N1, c0, c1, tw1, p0, H, pa.f_init, pa.f_stride)
             if (row_fs) {
                 if (pa.mode == PM_COMPLEX) {
                     if (n1 == 1024) NUDIM_ROWFS(PM_COMPLEX, 32, 32);
@@ -1589,14 +1602,12 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
                 }
             } else if (pa.mode == PM_COMPLEX)
 #undef NUDIM_ROWFS
-                k_rowfft<T, PM_COMPLEX><<<g, 256, smem_row, st>>>(pa.src, pa.src_stride, N0, N1,
-                                                                   n1, logn1, rows, c0, c1, tw1,
-                                                                   p0, H, nullptr, 0);
+                launch_early(k_rowfft<T, PM_COMPLEX>, g, 256, smem_row, st, pa.src, pa.src_stride,
+                             N0, N1, n1, logn1, rows, c0, c1, tw1, p0, H, nullptr, 0);
             else
-                k_rowfft<T, PM_REAL_INIT><<<g, 256, smem_row, st>>>(pa.src, pa.src_stride, N0,
-                                                                     N1, n1, logn1, rows, c0, c1,
-                                                                     tw1, p0, H, pa.f_init,
-                                                                     pa.f_stride);
+                launch_early(k_rowfft<T, PM_REAL_INIT>, g, 256, smem_row, st, pa.src,
+                             pa.src_stride, N0, N1, n1, logn1, rows, c0, c1, tw1, p0, H, pa.f_init,
+                             pa.f_stride);
             NUDIM_LAUNCH_CHECK();
         }
         {
@@ -1608,19 +1619,19 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             // one radix-16 butterfly per thread: 64 threads per column
             const int thr = std::min(32 * col_warps<T>(), std::max(64, 64 * BC));
 #define NUDIM_COLFS(R1, R2)                                                                      \
-    k_colfft_interp_fs<R1, R2><<<dim3(nc, nb), thr, smem_colfs_of<double>(R1, R2), st>>>(           \
-        (const double2 *)H, N0, n1, (const double2 *)tw0, cu, ent, e_rb, e_cc,                 \
+    launch_early(k_colfft_interp_fs<R1, R2>, dim3(nc, nb), thr, smem_colfs_of<double>(R1, R2), \
+        st, (const double2 *)H, N0, n1, (const double2 *)tw0, cu, ent, e_rb, e_cc, \
         (const double *)e_qa, (const double *)e_q1, nE, M, smax, (double2 *)P, Ew)
 #define NUDIM_COLFS2(R1, R2)                                                                     \
-    k_colfft_interp_fs2<R1, R2><<<dim3(nc, ceil_div(nb, 2)), 256,                             \
-                                  sizeof(float2) * 2 * 4 * fs2_gs<R1, R2>(), st>>>(             \
-        (const float2 *)H, N0, n1, nb, (const float2 *)tw0, cu, ent, e_rb, e_cc,            \
-        (const float *)e_qa, (const float *)e_q1, nE, M, smax, (float2 *)P)
+    launch_early(k_colfft_interp_fs2<R1, R2>, dim3(nc, ceil_div(nb, 2)), 256, \
+        sizeof(float2) * 2 * 4 * fs2_gs<R1, R2>(), st, (const float2 *)H, N0, n1, nb, \
+        (const float2 *)tw0, cu, ent, e_rb, e_cc, (const float *)e_qa, (const float *)e_q1, \
+        nE, M, smax, (float2 *)P)
 #define NUDIM_COLFS8(R1, R2)                                                                     \
-    k_colfft_interp_fs8<R1, R2><<<dim3(nc, nb), 256, sizeof(float2) * 8 * fs8_gs<R1, R2>(),    \
-                                  st>>>((const float2 *)H, N0, n1, (const float2 *)tw0, cu,      \
-                                        ent, e_rb, e_cc, (const float *)e_qa,                   \
-                                        (const float *)e_q1, nE, M, smax, (float2 *)P)
+    launch_early(k_colfft_interp_fs8<R1, R2>, dim3(nc, nb), 256, \
+        sizeof(float2) * 8 * fs8_gs<R1, R2>(), st, (const float2 *)H, N0, n1, \
+        (const float2 *)tw0, cu, ent, e_rb, e_cc, (const float *)e_qa, (const float *)e_q1, \
+        nE, M, smax, (float2 *)P)
             if (sizeof(T) == 4 && BC == 8 && n0 == 1024) NUDIM_COLFS8(32, 32);
             else if (sizeof(T) == 4 && BC == 8 && n0 == 512) NUDIM_COLFS8(32, 16);
             else if (sizeof(T) == 4 && BC == 8 && n0 == 256) NUDIM_COLFS8(16, 16);
@@ -1631,9 +1642,8 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             else if (BC == 4 && n0 == 512) NUDIM_COLFS(32, 16);
             else if (BC == 4 && n0 == 256) NUDIM_COLFS(16, 16);
             else
-                k_colfft_interp<T><<<dim3(nc, nb), thr, smem_col, st>>>(
-                    H, N0, n0, logn0, n1, BC, tw0, cu, ent, e_rb, e_cc, e_qa, e_q1, nE, M,
-                    smax, P, Ew);
+                launch_early(k_colfft_interp<T>, dim3(nc, nb), thr, smem_col, st, H, N0, n0, logn0,
+                             n1, BC, tw0, cu, ent, e_rb, e_cc, e_qa, e_q1, nE, M, smax, P, Ew);
 #undef NUDIM_COLFS
 #undef NUDIM_COLFS2
 #undef NUDIM_COLFS8
@@ -1643,10 +1653,14 @@ int NfftDev<T>::trafo_fused(int nplanes, const PadArgs<T> &pa, const InterpArgs<
             ProfScope ps(ctx, PK_CGVEC, st, nb * c * ((double)smax * M + M));
             dim3 g(interp_blocks(), nb);
             switch (ia.mode) {
-            case IM_PLAIN: k_combine<T, IM_PLAIN><<<g, 256, 0, st>>>(P, nslots, M, smax, p0, ia); break;
-            case IM_RESID: k_combine<T, IM_RESID><<<g, 256, 0, st>>>(P, nslots, M, smax, p0, ia); break;
-            case IM_DOTV: k_combine<T, IM_DOTV><<<g, 256, 0, st>>>(P, nslots, M, smax, p0, ia); break;
-            default: k_combine<T, IM_CONSTRAINT><<<g, 256, 0, st>>>(P, nslots, M, smax, p0, ia); break;
+            case IM_PLAIN: launch_early(k_combine<T, IM_PLAIN>, g, 256, 0, st, P, nslots, M, smax,
+                                        p0, ia); break;
+            case IM_RESID: launch_early(k_combine<T, IM_RESID>, g, 256, 0, st, P, nslots, M, smax,
+                                        p0, ia); break;
+            case IM_DOTV: launch_early(k_combine<T, IM_DOTV>, g, 256, 0, st, P, nslots, M, smax,
+                                       p0, ia); break;
+            default: launch_early(k_combine<T, IM_CONSTRAINT>, g, 256, 0, st, P, nslots, M, smax,
+                                  p0, ia); break;
             }
             NUDIM_LAUNCH_CHECK();
         }
@@ -1684,9 +1698,8 @@ int NfftDev<T>::adjoint_fused(int nplanes, const SpreadArgs<T> &sa, const CropAr
             dim3 g(ceil_div(nunits, upc), ceil_div(nb, Pl));
             const int thr = 32 * kGatherWarps;
 #define NUDIM_GATHER(WT, PP)                                                                    \
-    k_spread_gather<T, WT, PP><<<g, thr, smem_spread, st>>>(sa, units, nunits, upc, band_node,  \
-                                                            band_w, nbands, n0, n1, BCa, nb,    \
-                                                            p0, G, part, Ew)
+    launch_early(k_spread_gather<T, WT, PP>, g, thr, smem_spread, st, sa, units, nunits, upc, \
+        band_node, band_w, nbands, n0, n1, BCa, nb, p0, G, part, Ew)
             if (sa.w) {
                 if (Pl == 8) NUDIM_GATHER(true, 8);
                 else if (Pl == 4) NUDIM_GATHER(true, 4);
@@ -1701,8 +1714,8 @@ int NfftDev<T>::adjoint_fused(int nplanes, const SpreadArgs<T> &sa, const CropAr
 #undef NUDIM_GATHER
             NUDIM_LAUNCH_CHECK();
             if (nfix > 0) {
-                k_spread_fixup<T><<<dim3(nfix, ceil_div(nb, 8)), 256, 0, st>>>(
-                    fixups, nbands, n0, n1, BCa, nb, part, G);
+                launch_early(k_spread_fixup<T>, dim3(nfix, ceil_div(nb, 8)), 256, 0, st, fixups,
+                             nbands, n0, n1, BCa, nb, part, G);
                 NUDIM_LAUNCH_CHECK();
             }
         }
@@ -1713,21 +1726,25 @@ int NfftDev<T>::adjoint_fused(int nplanes, const SpreadArgs<T> &sa, const CropAr
                 (n0 == 1024 ? fs_col_stride<32, 32>() : n0 == 512 ? fs_col_stride<32, 16>()
                                                                   : fs_col_stride<16, 16>());
             if (BCa == 4 && n0 == 1024)
-                k_colifft_fs<T, 32, 32><<<dim3(nblka, nb), 128, smem_fs, st>>>(G, N0, n1, tw0, Hp);
+                launch_early(k_colifft_fs<T, 32, 32>, dim3(nblka, nb), 128, smem_fs, st, G, N0, n1,
+                             tw0, Hp);
             else if (BCa == 4 && n0 == 512)
-                k_colifft_fs<T, 32, 16><<<dim3(nblka, nb), 64, smem_fs, st>>>(G, N0, n1, tw0, Hp);
+                launch_early(k_colifft_fs<T, 32, 16>, dim3(nblka, nb), 64, smem_fs, st, G, N0, n1,
+                             tw0, Hp);
             else if (BCa == 4 && n0 == 256)
-                k_colifft_fs<T, 16, 16><<<dim3(nblka, nb), 64, smem_fs, st>>>(G, N0, n1, tw0, Hp);
+                launch_early(k_colifft_fs<T, 16, 16>, dim3(nblka, nb), 64, smem_fs, st, G, N0, n1,
+                             tw0, Hp);
             else
-                k_colifft<T><<<dim3(nblka, nb), 256, smem_colifft, st>>>(G, N0, n0, logn0, n1,
-                                                                          BCa, tw0, Hp);
+                launch_early(k_colifft<T>, dim3(nblka, nb), 256, smem_colifft, st, G, N0, n0,
+                             logn0, n1, BCa, tw0, Hp);
             NUDIM_LAUNCH_CHECK();
         }
         {
             ProfScope ps(ctx, PK_CROP, st, nb * c * ((double)N0 * n1 + 2.0 * N0 * N1));
             dim3 g(ceil_div(N0, rows), nb);
 #define NUDIM_CROPFS(MD, R1, R2)                                                                 \
-    k_rowifft_crop_fs<T, MD, R1, R2><<<g, 128, smem_row, st>>>(Hp, N0, N1, c0, c1, tw1, p0, ca)
+    launch_early(k_rowifft_crop_fs<T, MD, R1, R2>, g, 128, smem_row, st, Hp, N0, N1, c0, c1, \
+        tw1, p0, ca)
 #define NUDIM_CROPFS_N(MD)                                                                       \
     do {                                                                                        \
         if (n1 == 1024) NUDIM_CROPFS(MD, 32, 32);                                               \
@@ -1742,9 +1759,12 @@ int NfftDev<T>::adjoint_fused(int nplanes, const SpreadArgs<T> &sa, const CropAr
 #undef NUDIM_CROPFS_N
 #undef NUDIM_CROPFS
             switch (ca.mode) {
-            case CM_PLAIN: k_rowifft_crop<T, CM_PLAIN><<<g, 256, smem_row, st>>>(Hp, N0, N1, n1, logn1, rows, c0, c1, tw1, p0, ca); break;
-            case CM_DOT: k_rowifft_crop<T, CM_DOT><<<g, 256, smem_row, st>>>(Hp, N0, N1, n1, logn1, rows, c0, c1, tw1, p0, ca); break;
-            default: k_rowifft_crop<T, CM_INIT><<<g, 256, smem_row, st>>>(Hp, N0, N1, n1, logn1, rows, c0, c1, tw1, p0, ca); break;
+            case CM_PLAIN: launch_early(k_rowifft_crop<T, CM_PLAIN>, g, 256, smem_row, st, Hp, N0,
+                                        N1, n1, logn1, rows, c0, c1, tw1, p0, ca); break;
+            case CM_DOT: launch_early(k_rowifft_crop<T, CM_DOT>, g, 256, smem_row, st, Hp, N0, N1,
+                                      n1, logn1, rows, c0, c1, tw1, p0, ca); break;
+            default: launch_early(k_rowifft_crop<T, CM_INIT>, g, 256, smem_row, st, Hp, N0, N1, n1,
+                                  logn1, rows, c0, c1, tw1, p0, ca); break;
             }
             NUDIM_LAUNCH_CHECK();
         }

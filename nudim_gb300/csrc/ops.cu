@@ -9,10 +9,11 @@ namespace nudim {
 // dots[p*4 + 0/1]: |z|^2 ping-pong, dots[p*4 + 2]: v^H W v.
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_cg_update(cplx_t<T> *__restrict__ f, const cplx_t<T> *__restrict__ p, cplx_t<T> *__restrict__ r,
-            const cplx_t<T> *__restrict__ v, const double *__restrict__ dots, int cur, int N,
+k_cg_update(cplx_t<T> *f, const cplx_t<T> *p, cplx_t<T> *r,
+            const cplx_t<T> *v, const double *dots, int cur, int N,
             int M)
 {
+    await_last();
     // one FP64 division per block (FP64 is slow here), shared with the block
     __shared__ T s_alpha;
     int b = blockIdx.y;
@@ -37,9 +38,10 @@ k_cg_update(cplx_t<T> *__restrict__ f, const cplx_t<T> *__restrict__ p, cplx_t<T
 
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_cg_pupdate(cplx_t<T> *__restrict__ p, const cplx_t<T> *__restrict__ z,
-             const double *__restrict__ dots, int cur, int nxt, int N)
+k_cg_pupdate(cplx_t<T> *p, const cplx_t<T> *z,
+             const double *dots, int cur, int nxt, int N)
 {
+    await_last();
     __shared__ T s_beta;
     int b = blockIdx.y;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -158,7 +160,7 @@ int cgnr_run(NfftDev<T> &pl, int nplanes, const cplx_t<T> *y, const T *w, cplx_t
         {
             ProfScope ps(pl.ctx, PK_CGVEC, st, 3.0 * sizeof(C) * ((double)N + M) * nplanes);
             dim3 gu(ceil_div((long)N + M, 256), nplanes);
-            k_cg_update<T><<<gu, 256, 0, st>>>(f, b.p, b.r, b.v, b.dots, cur, N, M);
+            launch_early(k_cg_update<T>, gu, 256, 0, st, f, b.p, b.r, b.v, b.dots, cur, N, M);
             NUDIM_LAUNCH_CHECK();
         }
         // z = A^H W r, |z|^2
@@ -176,7 +178,7 @@ int cgnr_run(NfftDev<T> &pl, int nplanes, const cplx_t<T> *y, const T *w, cplx_t
         {
             ProfScope ps(pl.ctx, PK_CGVEC, st, 3.0 * sizeof(C) * (double)N * nplanes);
             dim3 gp(ceil_div(N, 256), nplanes);
-            k_cg_pupdate<T><<<gp, 256, 0, st>>>(b.p, b.z, b.dots, cur, nxt, N);
+            launch_early(k_cg_pupdate<T>, gp, 256, 0, st, b.p, b.z, b.dots, cur, nxt, N);
             NUDIM_LAUNCH_CHECK();
         }
         cur = nxt;

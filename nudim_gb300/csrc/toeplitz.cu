@@ -50,10 +50,11 @@ enum RowMode {
 // the spectra, 96 planes of 384 x 384 at 6.8 TB/s (116 us).
 template <typename T, int MODE, int R1, int R2>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 2)
-k_toep_rows(const void *__restrict__ src, cplx_t<T> *__restrict__ f, cplx_t<T> *__restrict__ p,
-            const cplx_t<T> *__restrict__ z, const double *__restrict__ dots, int N0, int N1,
-            const cplx_t<T> *__restrict__ tw, int plane0, cplx_t<T> *__restrict__ H)
+k_toep_rows(const void *src, cplx_t<T> *f, cplx_t<T> *p,
+            const cplx_t<T> *z, const double *dots, int N0, int N1,
+            const cplx_t<T> *__restrict__ tw, int plane0, cplx_t<T> *H)
 {
+    await_last();
     using C = cplx_t<T>;
     constexpr int nt = R1 * R2, RPC = 128 / R2, Q = R1 / 4;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -129,10 +130,11 @@ k_toep_rows(const void *__restrict__ src, cplx_t<T> *__restrict__ f, cplx_t<T> *
 // (z holds A^H W y, g = T f); otherwise z -= alpha g.  Partial |z|^2 per CTA.
 template <typename T, bool RESID, int R1, int R2>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 2)
-k_toep_irows(const cplx_t<T> *__restrict__ H, cplx_t<T> *__restrict__ z,
-             const double *__restrict__ dots, int N0, int N1, const cplx_t<T> *__restrict__ tw,
-             int plane0, double *__restrict__ part, int part_stride)
+k_toep_irows(const cplx_t<T> *H, cplx_t<T> *z,
+             const double *dots, int N0, int N1, const cplx_t<T> *__restrict__ tw,
+             int plane0, double *part, int part_stride)
 {
+    await_last();
     using C = cplx_t<T>;
     constexpr int nt = R1 * R2, RPC = 128 / R2;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -215,10 +217,11 @@ template <typename T, int R1, int R2> struct ColShape {
 
 template <typename T, int R1, int R2>
 __global__ void __launch_bounds__(4 * R1, sizeof(T) == 4 ? (R1 == 16 ? 10 : 5) : (R1 == 16 ? 4 : 2))
-k_toep_cols(cplx_t<T> *__restrict__ H, int N0, const cplx_t<T> *__restrict__ tw,
-            const T *__restrict__ khat, double *__restrict__ part, int part_stride, int plane0,
+k_toep_cols(cplx_t<T> *H, int N0, const cplx_t<T> *__restrict__ tw,
+            const T *__restrict__ khat, double *part, int part_stride, int plane0,
             bool dot)
 {
+    await_last();
     using C = cplx_t<T>;
     constexpr int nt = R1 * R2, RS = ColShape<T, R1, R2>::RS, CS = ColShape<T, R1, R2>::CS;
     constexpr int Q = R1 / 4, NT = 4 * R1;
@@ -326,9 +329,10 @@ k_toep_cols(cplx_t<T> *__restrict__ H, int N0, const cplx_t<T> *__restrict__ tw,
 // sum; 2 beta = sum / |z|^2 and the new |z|^2.
 template <typename T, int STEP>
 __global__ void __launch_bounds__(128)
-k_cg_scalar(const double *__restrict__ part, int nparts, int stride, int plane0,
-            double *__restrict__ dots)
+k_cg_scalar(const double *part, int nparts, int stride, int plane0,
+            double *dots)
 {
+    await_last();
     __shared__ double sh[32];
     const int gb = plane0 + blockIdx.x;
     const double *src = part + (size_t)gb * stride;
@@ -346,9 +350,10 @@ k_cg_scalar(const double *__restrict__ part, int nparts, int stride, int plane0,
 // f += alpha p after the last step
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_cg_last(cplx_t<T> *__restrict__ f, const cplx_t<T> *__restrict__ p,
-          const double *__restrict__ dots, int N, int plane0)
+k_cg_last(cplx_t<T> *f, const cplx_t<T> *p,
+          const double *dots, int N, int plane0)
 {
+    await_last();
     const int gb = plane0 + blockIdx.y;
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (size_t)N) return;
@@ -484,7 +489,8 @@ template <typename T, int R1, int R2> struct ToepLaunch {
             ProfScope ps(pl.ctx, PK_TOEPLITZ, st,
                          (mode == TR_CG ? 5 : mode == TR_COMPLEX ? 1 : 2) * v + h);
 #define NUDIM_ROWS(M)                                                                            \
-    k_toep_rows<T, M, R1, R2><<<g, 128, smem_row, st>>>(src, f, p, z, dots, N0, N1, pl.twT, p0, H)
+    launch_early(k_toep_rows<T, M, R1, R2>, g, 128, smem_row, st, src, f, p, z, dots, N0, N1, \
+        pl.twT, p0, H)
             if (mode == TR_COMPLEX) NUDIM_ROWS(TR_COMPLEX);
             else if (mode == TR_REAL) NUDIM_ROWS(TR_REAL);
             else if (mode == TR_FIRST) NUDIM_ROWS(TR_FIRST);
@@ -494,25 +500,28 @@ template <typename T, int R1, int R2> struct ToepLaunch {
         }
         {
             ProfScope ps(pl.ctx, PK_TOEPLITZ, st, 2 * h + sizeof(T) * (double)nt * nt);
-            k_toep_cols<T, C1, C2><<<dim3(nt / 4, nb), 4 * C1, smem_col, st>>>(
-                H, N0, pl.twT, pl.khat, part, part_stride, p0, !resid);
+            launch_early(k_toep_cols<T, C1, C2>, dim3(nt / 4, nb), 4 * C1, smem_col, st, H, N0,
+                         pl.twT, pl.khat, part, part_stride, p0, !resid);
             NUDIM_LAUNCH_CHECK();
             if (!resid) {
-                k_cg_scalar<T, 1><<<nb, 128, 0, st>>>(part, nt / 4, part_stride, p0, dots);
+                launch_early(k_cg_scalar<T, 1>, nb, 128, 0, st, part, nt / 4, part_stride, p0,
+                             dots);
                 NUDIM_LAUNCH_CHECK();
             }
         }
         {
             ProfScope ps(pl.ctx, PK_TOEPLITZ, st, h + 2 * v);
             if (resid)
-                k_toep_irows<T, true, R1, R2><<<g, 128, smem_row, st>>>(
-                    H, z, dots, N0, N1, pl.twT, p0, part, part_stride);
+                launch_early(k_toep_irows<T, true, R1, R2>, g, 128, smem_row, st, H, z, dots, N0,
+                             N1, pl.twT, p0, part, part_stride);
             else
-                k_toep_irows<T, false, R1, R2><<<g, 128, smem_row, st>>>(
-                    H, z, dots, N0, N1, pl.twT, p0, part, part_stride);
+                launch_early(k_toep_irows<T, false, R1, R2>, g, 128, smem_row, st, H, z, dots, N0,
+                             N1, pl.twT, p0, part, part_stride);
             NUDIM_LAUNCH_CHECK();
-            if (resid) k_cg_scalar<T, 0><<<nb, 128, 0, st>>>(part, (int)g.x, part_stride, p0, dots);
-            else k_cg_scalar<T, 2><<<nb, 128, 0, st>>>(part, (int)g.x, part_stride, p0, dots);
+            if (resid) launch_early(k_cg_scalar<T, 0>, nb, 128, 0, st, part, (int)g.x, part_stride,
+                                    p0, dots);
+            else launch_early(k_cg_scalar<T, 2>, nb, 128, 0, st, part, (int)g.x, part_stride, p0,
+                              dots);
             NUDIM_LAUNCH_CHECK();
         }
         return NUDIM_OK;
@@ -659,7 +668,8 @@ int NfftDev<T>::toeplitz_cg(int nplanes, C *f, const T *f_real, bool f_zero, int
     for (int p0 = 0; p0 < nplanes; p0 += chunk) {
         const int nb = std::min(chunk, nplanes - p0);
         if (f_zero) {
-            k_cg_scalar<T, 0><<<nb, 128, 0, st>>>(part, crop_blocks(), part_stride, p0, dots);
+            launch_early(k_cg_scalar<T, 0>, nb, 128, 0, st, part, crop_blocks(), part_stride, p0,
+                         dots);
             NUDIM_LAUNCH_CHECK();
         } else {
             NUDIM_TRY(pass(f_real ? TR_REAL : TR_COMPLEX, true, p0, nb));
@@ -667,7 +677,7 @@ int NfftDev<T>::toeplitz_cg(int nplanes, C *f, const T *f_real, bool f_zero, int
         for (int it = 0; it < iters; it++) NUDIM_TRY(pass(it ? TR_CG : TR_FIRST, false, p0, nb));
         if (iters > 0) {
             ProfScope ps(ctx, PK_CGVEC, st, 3.0 * sizeof(C) * (double)N * nb);
-            k_cg_last<T><<<dim3(ceil_div(N, 256), nb), 256, 0, st>>>(f, p, dots, N, p0);
+            launch_early(k_cg_last<T>, dim3(ceil_div(N, 256), nb), 256, 0, st, f, p, dots, N, p0);
             NUDIM_LAUNCH_CHECK();
         }
     }
