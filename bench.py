@@ -217,28 +217,26 @@ def timed_steps(ctx, job, steps, nvtx=None):
 MEASURED_ADJOINT_TRAFFIC_PER_PLANE = ((172.924160e6 + 216.713216e6)    # k_spread_gather
                                       + (268.486656e6 + 75.897088e6)   # k_colifft_fs
                                       + (100.737792e6 + 36.037120e6)) / 32  # k_rowifft_crop
-# The same for the Toeplitz operator pass (k_rowfft_fs + k_col_toeplitz +
-# k_rowifft_crop_fs in its p^H q mode) per circulant size, 32-plane launches:
-# the row spectra between the passes stay partly in the 129 MB L2 at that size.
+# The same for a step of the Toeplitz CG (k_toep_rows + k_toep_cols +
+# k_toep_irows) on the 768-point circulant, 32-plane launches: the row spectra
+# between the passes stay partly in the 129 MB L2 at that size.
 MEASURED_TOEPLITZ_TRAFFIC_PER_PLANE = {
-    768: ((37.8e6 + 15.6e6)                 # k_rowfft_fs<.., 24, 32>
-          + (80.3e6 + 17.5e6)               # k_col_toeplitz<.., 24, 32>
-          + (113.3e6 + 13.4e6)) / 32,       # k_rowifft_crop_fs<.., 24, 32>
-    1024: ((37.8e6 + 36.6e6)                # k_rowfft_fs
-           + (109.1e6 + 42.6e6)             # k_col_toeplitz
-           + (138.5e6 + 15.6e6)) / 32,      # k_rowifft_crop_fs
+    768: ((113.28e6 + 89.35e6)              # k_toep_rows<.., 3, 24, 32>
+          + (77.90e6 + 17.22e6)             # k_toep_cols<.., 32, 24>
+          + (113.28e6 + 12.71e6)) / 32,     # k_toep_irows<.., 0, 24, 32>
 }
 
 
 def roofline_from_profile(prof, peak_gbs, peak_kind, r, csize, steps):
     """Roofline of the dominant kernel group of the mixed form's iteration.
 
-    - The Toeplitz operator pass of the CGNR (k_rowfft_fs + k_col_toeplitz +
-      k_rowifft_crop_fs, class "toeplitz"): 11 per Z-plane and outer
-      iteration (one before the loop, one per step).  Unit: one Z-plane's
-      pass, c (3 P^2 + 4 P nt) bytes -- p in, T p out and p read again for
-      p^H T p, and the P x nt row spectra written, read and written by the
-      column pass, and read back (nt: the circulant's size, 768 for P = 384).
+    - The Toeplitz CG's passes (k_toep_rows + k_toep_cols + k_toep_irows,
+      class "toeplitz"): 11 per Z-plane and outer iteration (one before the
+      loop, one per step).  Unit: one Z-plane's operator pass, c (3 P^2 +
+      4 P nt) bytes -- p in, T p out and p read again for p^H T p, and the
+      P x nt row spectra written, read and written by the column pass, and
+      read back (nt: the circulant's size, 768 for P = 384).  The vector
+      updates that ride on the row passes (another 4 P^2) are not counted.
     - The adjoint NFFT (k_spread_gather + k_spread_fixup + k_colifft_fs +
       k_rowifft_crop_fs, classes "spread" + "crop"): 11 per Z-plane and outer
       iteration with the NFFT form of the CGNR, 1 with the Toeplitz form.
@@ -260,7 +258,7 @@ def roofline_from_profile(prof, peak_gbs, peak_kind, r, csize, steps):
         unit = csize * (3 * P * P + 4 * P * nt)
         tr = MEASURED_TOEPLITZ_TRAFFIC_PER_PLANE.get(nt)
         groups.append(("Toeplitz operator pass",
-                       "Toeplitz operator pass (k_rowfft_fs + k_col_toeplitz + k_rowifft_crop_fs)",
+                       "Toeplitz CG step (k_toep_rows + k_toep_cols + k_toep_irows)",
                        toep[0], units, launches, unit, tr))
     ms_s, n_s, _ = prof["spread"]
     ms_c, n_c, _ = prof["crop"]
