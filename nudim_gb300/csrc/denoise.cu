@@ -132,16 +132,10 @@ template <> struct TvNorm<double> {
 template <typename T> struct TvAcc;
 template <> struct TvAcc<double> {
     double g = 0, n = 0;
-    static __device__ __forceinline__ double square(double a)
-    {
-        double q;
-        if (!int_square(a, &q)) q = rn_mul(a, a);
-        return q;
-    }
     __device__ __forceinline__ void add_sq(double a, double b)
     {
-        g = rn_add(g, square(a));
-        n = rn_add(n, square(b));
+        g = rn_add(g, square_rn(a));
+        n = rn_add(n, square_rn(b));
     }
     __device__ __forceinline__ double grad() const { return g; }
     __device__ __forceinline__ double neg() const { return n; }

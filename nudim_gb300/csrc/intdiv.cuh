@@ -269,6 +269,22 @@ NUDIM_HD bool int_square(double z, double *out)
     return e < 1023 + 500;
 }
 
+// RN(z z) for any z: what int_square leaves (near overflow) or flushes (below
+// 2^-998: harmless under the norm's 1e-8, but a sum of such squares is not 0)
+// is the FP64 unit's.
+NUDIM_HD double square_rn(double z)
+{
+    double q;
+    if (!int_square(z, &q) || (!bits_of(q) && bits_of(z) << 1)) {
+#if defined(__CUDA_ARCH__)
+        q = __dmul_rn(z, z);
+#else
+        q = z * z;
+#endif
+    }
+    return q;
+}
+
 // RN(sqrt(s)) for a positive normal s, as a divisor.  With s = d 4^h, d in [1/4,
 // 1): y0 ~ 1 / sqrt(d) from the FP32 seed, one Newton step (within 2^-42), then
 // the square root from the 48 leading bits n1 of d y1 and the exact residual
