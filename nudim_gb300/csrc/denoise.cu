@@ -206,8 +206,8 @@ __device__ __forceinline__ double tv_root(double s)
 // k_tv_update's operations), the owned cells' u' are written to u_out and the gradient of u' to g: one pass reads u and g_in and
 // writes u' and g (4 values per voxel instead of the 5 of a gradient and an
 // update).  u_out and g must not alias u and g_in (other blocks still read
-// their halos).
-template <typename T, bool FUSED>
+// their halos).  I: the index within a plane.
+template <typename T, bool FUSED, typename I>
 __global__ void __launch_bounds__(256, kTvSumBlocks<T>)
 k_tv_grad(const T *u, T *g, double *part,
           unsigned *done, double *step, int nz, int ny, int nx,
@@ -237,16 +237,16 @@ k_tv_grad(const T *u, T *g, double *part,
         own[r] = inb[r] && (!height || (j >= ylo && j <= yhi));
     }
     const size_t P = (size_t)ny * nx;
-    const unsigned my = (unsigned)(j0 + ty) * nx + k, my8 = my + 8u * nx;  // this thread's voxels
+    const I my = (I)(j0 + ty) * nx + k, my8 = my + (I)8 * nx;  // this thread's voxels
     // this thread's halo-tile cells (threadIdx + 256 s), their clamped in-plane
     // offsets and (FUSED) whether the update applies to their row
-    unsigned off[kSlots];
+    I off[kSlots];
     bool upd[kSlots];
 #pragma unroll
     for (int s = 0; s < kSlots; s++) {
         const int c = threadIdx.x + 256 * s, yy = c / kTvSX, xx = c - yy * kTvSX;
         const int gj = min(max(j0 + yy - 1, 0), ny - 1), gk = min(max(k0 + xx - 1, 0), nx - 1);
-        off[s] = (unsigned)gj * nx + gk;
+        off[s] = (I)gj * nx + gk;
         upd[s] = c < kCells && (!height || (gj >= ylo && gj <= yhi));
     }
     T la = T(0);
@@ -515,7 +515,8 @@ template <typename T> static bool tv_unfused()
     return sizeof(T) == 8;
 }
 
-template <typename T, typename I>
+// I: the index of a voxel in the volume; G: within a plane
+template <typename T, typename I, typename G>
 static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, size_t V, int nz,
                      int ny, int nx, float lam, int niter, int height, int ylo, int yhi,
                      T *u2, T *g2, cudaStream_t st)
@@ -567,7 +568,7 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     if (niter <= 0) return NUDIM_OK;
     if (!u2 || !g2 || niter < 2 || tv_unfused<T>()) {
         for (int it = 0; it < niter; it++) {
-            k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc,
+            k_tv_grad<T, false, G><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc,
                                                     runs, rep, height, ylo, yhi, nullptr, nullptr,
                                                     (double)lam, nullptr);
             NUDIM_LAUNCH_CHECK();
@@ -579,7 +580,7 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     // previous gradient and take the next one (volumes and gradients alternate
     // between (u, grad) and (u2, g2), the sums between scal[0..1] and
     // scal[2..3]), then the last update into u
-    k_tv_grad<T, false><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc, runs, rep,
+    k_tv_grad<T, false, G><<<gg, 256, 0, st>>>(u, grad, part, done, scal, nz, ny, nx, zc, runs, rep,
                                             height, ylo, yhi, nullptr, nullptr, (double)lam, nullptr);
     NUDIM_LAUNCH_CHECK();
     T *cu = u, *cg = grad;
@@ -587,7 +588,7 @@ static int tv_launch(T *u, T *grad, double *part, int part_cap, double *scal, si
     for (int it = 1; it < niter; it++) {
         T *nu = cu == u ? u2 : u, *ng = cg == grad ? g2 : grad;
         double *ns = cs == scal ? scal + 2 : scal;
-        launch_early(k_tv_grad<T, true>, gg, 256, 0, st, cu, ng, part, done, ns, nz, ny, nx, zc,
+        launch_early(k_tv_grad<T, true, G>, gg, 256, 0, st, cu, ng, part, done, ns, nz, ny, nx, zc,
                      runs, rep, height, ylo, yhi, cg, cs, (double)lam, nu);
         NUDIM_LAUNCH_CHECK();
         cu = nu;
@@ -603,12 +604,14 @@ int tv_run(T *u, T *grad, double *part, int part_cap, double *scal, int nz, int 
 {
     size_t V = (size_t)nz * ny * nx;
     if (V == 0 || niter <= 0) return NUDIM_OK;
-    // 32-bit voxel indices while index + grid stride stays below 2^32
-    if (V < ((size_t)1 << 31))
-        return tv_launch<T, unsigned>(u, grad, part, part_cap, scal, V, nz, ny, nx, lam, niter,
-                                      height, ylo, yhi, u2, g2, st);
-    return tv_launch<T, size_t>(u, grad, part, part_cap, scal, V, nz, ny, nx, lam, niter, height,
-                                ylo, yhi, u2, g2, st);
+    // 32-bit voxel indices while index + grid stride stays below 2^32, within a
+    // plane while the plane does
+    const bool plane32 = (size_t)ny * nx <= ((size_t)1 << 32);
+    auto run = V < ((size_t)1 << 31) ? tv_launch<T, unsigned, unsigned>
+               : plane32             ? tv_launch<T, size_t, unsigned>
+                                     : tv_launch<T, size_t, size_t>;
+    return run(u, grad, part, part_cap, scal, V, nz, ny, nx, lam, niter, height, ylo, yhi, u2, g2,
+               st);
 }
 
 // ================================================================ diffusion
