@@ -45,7 +45,7 @@ template <typename T> StripShape strip_shape(int nz, int ny, int nx, int left, i
     s.C = 1;
     if (sizeof(T) == 8) {
         s.Q = 1;
-        auto turns = [&](int c) { return (nz * c + sms - 1) / sms; };
+        auto turns = [&](long long c) { return (nz * c + sms - 1) / sms; };
         for (int c = 2; c <= 8 && 2 * c <= left; c *= 2)
             if (turns(c) * s.C < turns(s.C) * c) s.C = c;
         const int most = s.C == 8 && turns(8) == 1 && left >= 40 ? 40 : 16;
@@ -56,7 +56,7 @@ template <typename T> StripShape strip_shape(int nz, int ny, int nx, int left, i
                 break;
             }
         s.k = s.W * s.C;
-    } else if (s.B == 1 && s.R >= 6 && 4 * nz <= sms && left >= 40) {
+    } else if (s.B == 1 && s.R >= 6 && nz <= sms / 4 && left >= 40) {
         s.C = 4;
         s.k = 40;
         s.Q = 1;
@@ -74,6 +74,15 @@ template <typename T> StripShape strip_shape(int nz, int ny, int nx, int left, i
     const int per = std::max(1, 16 / (s.W * s.B));  // CTAs an SM holds (128 registers)
     s.clusters = std::max(1, std::min(nz, sms * per / s.C));
     return s;
+}
+
+// Rounds of the next launch, k sweeps each.  The kernel counts a launch's steps
+// and diagonals, rounds P + nx + ny + 2 k of them, in 32 bits.
+constexpr int kStripsMaxNx = 1 << 28;
+inline int strip_rounds(const StripShape &s, int ny, int nx, int left)
+{
+    const long long most = ((1ll << 30) - nx - ny - 2 * s.k) / s.P;
+    return (int)std::min<long long>(left / s.k, most);
 }
 
 }  // namespace nudim

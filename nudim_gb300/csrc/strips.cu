@@ -505,7 +505,7 @@ int launch_rows(const StripShape &s, T *u, T *S, int *flags, const StripArgs<T> 
 template <typename T>
 bool strips_fits(int ny, int nx, int niter, double lambda, double ksq)
 {
-    if (ny < 1 || nx < 1 || ny > kBandRows<T> * 16 || niter < 1) return false;
+    if (ny < 1 || nx < 1 || nx > kStripsMaxNx || ny > kBandRows<T> * 16 || niter < 1) return false;
     CellArgs<T> c;
     if (sizeof(T) == 8) return cell_args(lambda, ksq, &c);
     return ksq >= kMinKsq && ksq <= kMaxKsq &&
@@ -519,7 +519,7 @@ template <typename T> size_t strips_scratch(int nz, int ny, int nx, int niter)
     for (int left = niter; left > 0;) {
         const StripShape s = strip_shape<T>(nz, ny, nx, left, sm_count());
         most = std::max(most, sizeof(T) * (size_t)s.clusters * s.P * 32 * s.R * s.B);
-        left -= left / s.k * s.k;
+        left -= strip_rounds(s, ny, nx, left) * s.k;
     }
     return most + strips_flag_bytes(nz);
 }
@@ -538,7 +538,7 @@ int strips_run(T *u, int nz, int ny, int nx, int nxb, double lambda, double ksq,
     if (sizeof(T) == 4) NUDIM_CUDA(cudaMemsetAsync(flags, 0, strips_flag_bytes(nz), st));
     for (int left = niter; left > 0;) {
         const StripShape s = strip_shape<T>(nz, ny, nx, left, sm_count());
-        const int rounds = left / s.k;
+        const int rounds = strip_rounds(s, ny, nx, left);
         a.nz = nz;
         a.ny = ny;
         a.nx = nx;

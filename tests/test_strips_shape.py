@@ -26,6 +26,11 @@ extern "C" void shape_of(int fp64, int nz, int ny, int nx, int left, int sms, in
     if (fp64) shape<double>(nz, ny, nx, left, sms, o);
     else shape<float>(nz, ny, nx, left, sms, o);
 }
+extern "C" int rounds_of(int fp64, int nz, int ny, int nx, int left, int sms)
+{
+    return nudim::strip_rounds(fp64 ? nudim::strip_shape<double>(nz, ny, nx, left, sms)
+                                    : nudim::strip_shape<float>(nz, ny, nx, left, sms), ny, nx, left);
+}
 """
 
 
@@ -43,12 +48,14 @@ def shape_of(tmp_path_factory):
     so = str(d / "s.so")
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", inc, str(d / "s.cpp"),
                     "-o", so], check=True)
-    fn = ctypes.CDLL(so).shape_of
+    lib = ctypes.CDLL(so)
 
     def get(fp64, nz, ny, nx, left, sms=152):
         o = (ctypes.c_int * 8)()
-        fn(fp64, nz, ny, nx, left, sms, o)
-        return Shape(o)
+        lib.shape_of(fp64, nz, ny, nx, left, sms, o)
+        s = Shape(o)
+        s.rounds = lib.rounds_of(fp64, nz, ny, nx, left, sms)
+        return s
     return get
 
 
@@ -69,6 +76,23 @@ def test_shapes_hold_what_the_kernel_needs(shape_of, fp64, nz):
         for ny in [3073, 3200, 5000, 6144]:
             s = shape_of(0, nz, ny, 6, 80)
             assert s.k == 2 and s.P >= s.R
+
+
+@pytest.mark.parametrize("fp64", [0, 1])
+@pytest.mark.parametrize("ny,nx,niter", [(32, 100000, 400000), (2, 1 << 28, 100), (400, 5000, 2 ** 31 - 1),
+                                         (1, 1, 2 ** 31 - 1), (64, 384, 80), (33, 100, 47)])
+def test_steps_of_a_launch_fit_32_bits(shape_of, fp64, ny, nx, niter):
+    """Many sweeps of wide planes go in several launches, of all sweeps together;
+    the usual counts in as many launches as they have shapes."""
+    left, launches = niter, 0
+    while left:
+        s = shape_of(fp64, 1, ny, nx, left)
+        assert s.rounds >= 1
+        assert s.rounds * s.P + nx + ny + 2 * s.k < 2 ** 31
+        left -= s.rounds * s.k
+        launches += 1
+        assert left >= 0
+    assert launches <= (3 if niter < 100 and nx < 1000 else 20000)
 
 
 def masked(v, lam, kap, s, rounds, nxb):
@@ -120,8 +144,8 @@ def test_masks_at_the_header_s_shapes(shape_of, fp64, ny, nx, left, nxb):
     with np.errstate(invalid="ignore"):
         while n:
             s = shape_of(fp64, 1, ny, nx, n)
-            out = masked(out, 0.25, 0.005, s, n // s.k, nxb)
-            n -= n // s.k * s.k
+            out = masked(out, 0.25, 0.005, s, s.rounds, nxb)
+            n -= s.rounds * s.k
     assert np.array_equal(out, sequential(v, 0.25, 0.005, left, nxb))
 
 
