@@ -126,6 +126,14 @@ static int exp_field(double x)  // of a positive normal x
     return e + 1022;
 }
 
+// FP64 window sums in integers, or on the FP64 unit (NUDIM_FP64_SUMS=fp64; read
+// when a plan is made)
+static bool fp64_int_sums()
+{
+    const char *e = getenv("NUDIM_FP64_SUMS");
+    return !(e && !strcmp(e, "fp64"));
+}
+
 // weights to fixed point in place
 __global__ void __launch_bounds__(256) k_fix_weights(double *w, size_t n, int Ew)
 {
@@ -133,43 +141,71 @@ __global__ void __launch_bounds__(256) k_fix_weights(double *w, size_t n, int Ew
     if (i < n) *reinterpret_cast<Fixed *>(w + i) = to_fixed(w[i], Ew);
 }
 
-// The column block's values (cnt of them) to fixed point in place (all threads).
-// Returns their exponent field, or -1 where they stay FP64.
-__device__ __forceinline__ int fix_columns(double2 *G, int cnt, int Ew, int *sh)
+// The column block's values to fixed point in place (all threads): n rows of BC
+// columns, column stride `stride`, each group of kFixRows rows under its own
+// exponent field she[group]. Groups, because a block's rows reach from the
+// spectrum's peak to its far end: under one bound for all, the far nodes' sums
+// lost bits that FP64 sums keep. Returns whether it was done, or the values are
+// still FP64.
+constexpr int kFixRows = 16, kFixGroups = 256;
+__device__ __forceinline__ bool fix_columns(double2 *G, int stride, int n, int BC, int Ew, int *she)
 {
-    int E = 0;
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x)
-        E = max(E, max(exp_of(G[i].x), exp_of(G[i].y)));
-    E = __reduce_max_sync(0xffffffffu, E);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = E;
-    __syncthreads();
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) E = max(E, sh[w]);
-    if (!Ew || !fixed_range(E)) return -1;
-    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
-        const FixedC v{to_fixed(G[i].x, E), to_fixed(G[i].y, E)};
-        *reinterpret_cast<FixedC *>(G + i) = v;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    bool bad = !Ew;
+    for (int g = threadIdx.x >> 5; g * kFixRows < n; g += nw) {
+        int E = 0;
+        for (int k = lane; k < kFixRows * BC; k += 32) {
+            const int row = g * kFixRows + k % kFixRows;
+            if (row < n) {
+                const double2 v = G[(size_t)(k / kFixRows) * stride + row];
+                E = max(E, max(exp_of(v.x), exp_of(v.y)));
+            }
+        }
+        E = __reduce_max_sync(0xffffffffu, E);
+        if (lane == 0) she[g] = E;
+        bad |= !fixed_range(E);
+    }
+    if (__syncthreads_or(bad)) return false;
+    for (int g = threadIdx.x >> 5; g * kFixRows < n; g += nw) {
+        const int E = she[g];
+        for (int k = lane; k < kFixRows * BC; k += 32) {
+            const int row = g * kFixRows + k % kFixRows;
+            if (row < n) {
+                double2 *p = G + (size_t)(k / kFixRows) * stride + row;
+                const FixedC v{to_fixed(p->x, E), to_fixed(p->y, E)};
+                *reinterpret_cast<FixedC *>(p) = v;
+            }
+        }
     }
     __syncthreads();
-    return E;
+    return true;
 }
 
 // A node's window over the block's columns in the FP64 form: row weights as
 // fixed point (exponent field Ew), column q of the entry at gp(q). The rows are
 // summed in integers, the columns in FP64 (those in integers too: as long, and an
-// error up to twice as large).
+// error up to twice as large). The window's 14 rows lie in at most two groups: the
+// weights of the one with the smaller values are shifted to the other's field.
 template <typename F>
 __device__ __forceinline__ double2 window_fp64(const double *__restrict__ qa,
                                                const double *__restrict__ q1, size_t nE, int e,
-                                               int odd, int rb, int m0, int cnt, int Ew, int Ev,
-                                               F gp)
+                                               int odd, int rb, int m0, int cnt, int Ew, bool ints,
+                                               const int *she, F gp)
 {
     // the window's 14 rows (the 16 weights start at the even row below)
     qa += odd * nE + e;
     double ar = 0, ai = 0;
-    if (Ev >= 0) {
+    if (ints) {
         Fixed w[14];
 #pragma unroll
         for (int i = 0; i < 14; i++) w[i] = *reinterpret_cast<const Fixed *>(qa + i * nE);
+        const int r0 = (rb + odd) & m0, here = kFixRows - r0 % kFixRows;  // rows of the first group
+        const int Ea = she[r0 / kFixRows], Eb = she[((r0 + 13) & m0) / kFixRows];
+        const int E = max(Ea, Eb);
+        if (Ea != Eb) {
+#pragma unroll
+            for (int i = 0; i < 14; i++) w[i] = fixed_shift(w[i], E - (i < here ? Ea : Eb));
+        }
         for (int q = 0; q < cnt; q++) {
             const FixedC *g = reinterpret_cast<const FixedC *>(gp(q));
             FixedSum s;
@@ -180,7 +216,7 @@ __device__ __forceinline__ double2 window_fp64(const double *__restrict__ qa,
             ar = fma(w1, s.re(), ar);
             ai = fma(w1, s.im(), ai);
         }
-        const double sc = fixed_scale(Ew, Ev);
+        const double sc = fixed_scale(Ew, E);
         return make_double2(ar * sc, ai * sc);
     }
     for (int q = 0; q < cnt; q++) {
@@ -317,11 +353,9 @@ k_colfft_interp(const cplx_t<T> *H, int N0, int n0, int logn0, int n1, int BC,
     }
     __syncthreads();
     C *G = block_fft<T, -1>(A, B, n0, logn0, BC, tw0);
-    int Ev = 0;
-    if constexpr (sizeof(T) == 8) {
-        __shared__ int she[32];
-        Ev = fix_columns(G, BC * n0, Ew, she);
-    }
+    __shared__ int she[sizeof(T) == 8 ? kFixGroups : 1];
+    bool ints = false;
+    if constexpr (sizeof(T) == 8) ints = fix_columns(G, n0, n0, BC, Ew, she);
     const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
@@ -329,7 +363,7 @@ k_colfft_interp(const cplx_t<T> *H, int N0, int n0, int logn0, int n1, int BC,
         const int cl0 = ccn & 255, cnt = (ccn >> 8) & 255;
         if constexpr (sizeof(T) == 8) {
             part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] =
-                window_fp64(e_qa, e_q1, nE, e, ccn >> 16, rb, m0, cnt, Ew, Ev, [&](int q) {
+                window_fp64(e_qa, e_q1, nE, e, ccn >> 16, rb, m0, cnt, Ew, ints, she, [&](int q) {
                     return G + (size_t)((cl0 + q) & (BC - 1)) * n0;
                 });
         } else {
@@ -415,19 +449,16 @@ k_colfft_interp_fs(const double2 *H, int N0, int n1,
             for (int k2 = 0; k2 < R2; k2++) Gs[c * GS + k1 + R1 * k2] = y[fs_out<R2>(k2)];
         }
     }
-    // (the columns' padding, which fix_columns passes over)
-    for (int i = threadIdx.x; i < BC * (GS - n0); i += blockDim.x)
-        Gs[(i / (GS - n0)) * GS + n0 + i % (GS - n0)] = mkc<T>(0, 0);
     __syncthreads();
-    __shared__ int she[32];
-    const int Ev = fix_columns(Gs, BC * GS, Ew, she);
+    __shared__ int she[kFixGroups];
+    const bool ints = fix_columns(Gs, GS, n0, BC, Ew, she);
     const int beg = un.y, end = un.z;
     const int m0 = n0 - 1;
     for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
         const int js = ent[e], rb = e_rb[e], ccn = e_cc[e];
         const int cl0 = ccn & 255, cnt = (ccn >> 8) & 255;
         part[((size_t)b * smax + (js & 7)) * M + (js >> 3)] =
-            window_fp64(e_qa, e_q1, nE, e, ccn >> 16, rb, m0, cnt, Ew, Ev,
+            window_fp64(e_qa, e_q1, nE, e, ccn >> 16, rb, m0, cnt, Ew, ints, she,
                         [&](int q) { return Gs + (size_t)((cl0 + q) & (BC - 1)) * GS; });
     }
 }
@@ -1449,7 +1480,9 @@ template <typename T> int NfftDev<T>::init_fused(const NfftTables &t, cudaStream
             finite = finite && std::isfinite(v);
             m = std::max(m, std::fabs(v));
         }
-        Ew = finite && m > 1e-30 && m < 1e30 ? exp_field(m) : 0;
+        Ew = fp64_int_sums() && n0 <= kFixRows * kFixGroups && finite && m > 1e-30 && m < 1e30
+                 ? exp_field(m)
+                 : 0;
         const size_t na = L.ent_qa.size(), nw = L.band_w.size();
         if (Ew && na) k_fix_weights<<<ceil_div(na, 256), 256, 0, st>>>(e_qa, na, Ew);
         if (Ew && nw) k_fix_weights<<<ceil_div(nw, 256), 256, 0, st>>>(band_w, nw, Ew);
