@@ -293,7 +293,14 @@ int nudim_tv_noalloc(int precision, void *vol, int nz, int ny, int nx, float lam
 /* aniso_diffusion_2d (denoise.c:320-378), in place, Gauss-Seidel order per
  * Z-plane.  nx_bound is the value the reference compares the column index
  * with (its "nx" argument, the number of Z-planes in reconstruction.c:627);
- * a read one past the row is defined as 0.0. */
+ * a read one past the row is defined as 0.0.
+ * The call takes scratch (at most a copy of the volume with its planes padded
+ * to multiples of 64 rows and to 36 columns) from a stream-ordered pool of the
+ * context, in the order of `stream`, so that calls on several streams share
+ * nothing; up to 512 MB stay with the pool until nudim_ctx_destroy.  Without it -- the
+ * allocation fails, or `stream` is being captured, where the call allocates
+ * nothing -- the call runs the forms that need none: slower, FP64 results
+ * the same bit for bit, FP32 results with other roundings. */
 int nudim_diffusion2d(nudim_ctx *ctx, int precision, void *vol, int nz, int ny, int nx,
                       int nx_bound, float lambda, float kappa, int niter, void *stream);
 

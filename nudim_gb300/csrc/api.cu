@@ -1539,18 +1539,23 @@ int nudim_diffusion2d(nudim_ctx *ctx, int precision, void *vol, int nz, int ny, 
     NUDIM_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
     // scratch from the context's stream-ordered pool; without room for it the
-    // forms that need none run
-    const size_t nb = precision == NUDIM_FP64
+    // forms that need none run, and while the stream is captured (a graph with
+    // allocations can be instantiated once only and embedded nowhere)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        cap = cudaStreamCaptureStatusInvalidated;
+    }
+    const size_t nb = cap != cudaStreamCaptureStatusNone ? 0
+                      : precision == NUDIM_FP64
                           ? diffusion_scratch<double>(nz, ny, nx, lambda, kappa, niter)
                           : diffusion_scratch<float>(nz, ny, nx, lambda, kappa, niter);
     void *scr = nullptr;
-    if (nb) {
-        cudaMemPool_t pool;
-        NUDIM_TRY(ctx_pool(ctx, &pool));
-        if (cudaMallocFromPoolAsync(&scr, nb, pool, st) != cudaSuccess) {
-            cudaGetLastError();
-            scr = nullptr;
-        }
+    cudaMemPool_t pool;
+    if (nb && (ctx_pool(ctx, &pool) != NUDIM_OK ||
+               cudaMallocFromPoolAsync(&scr, nb, pool, st) != cudaSuccess)) {
+        cudaGetLastError();
+        scr = nullptr;
     }
     const int rc =
         precision == NUDIM_FP64
