@@ -94,7 +94,7 @@ template <typename T> struct JobState {
     C *data = nullptr, *y = nullptr, *r = nullptr, *v = nullptr, *z = nullptr, *p = nullptr,
       *slices = nullptr;
     int *known = nullptr;
-    void *diff = nullptr;  // diffusion scratch
+    void *diff = nullptr;  // diffusion scratch: z, r or its own
     double *part = nullptr, *dots = nullptr, *tv_part = nullptr, *tv_scal = nullptr,
            *rh = nullptr;
     int part_stride = 0, tv_cap = 0;
@@ -226,6 +226,13 @@ static float job_lambda(const nudim_job_desc &d)
 constexpr float kJobKappa = 0.005f;
 constexpr int kJobSweeps = 80;
 
+// whether a job state's diffusion scratch of db bytes needs a buffer of its own,
+// beside the CGNR vectors z (V complex values) and r (S: planes x nodes)
+template <typename T> static bool diffusion_own(size_t db, size_t V, size_t S)
+{
+    return db > std::max(V, S) * sizeof(cplx_t<T>);
+}
+
 // The CGNR form of a job state: NFFT (a trafo and an adjoint per step, the
 // reference's own route and the FP64 default) or Toeplitz (one convolution
 // pass per step, the FP32 default where the plan's grid allows it);
@@ -296,10 +303,12 @@ template <typename T> static int state_init(nudim_job *jb, JobState<T> &s)
         NUDIM_TRY(s.alloc(&s.tv_scal, 4));
     }
     if (jb->d.denoise == NUDIM_DENOISE_DIFFUSION) {
+        // the CGNR vectors z and r (rewritten by every CGNR run) are free while
+        // the diffusion runs
         const size_t db = diffusion_scratch<T>(nz, np, np, job_lambda(jb->d), kJobKappa, kJobSweeps);
-        char *q = nullptr;
-        if (db) NUDIM_TRY(s.alloc(&q, db));
-        s.diff = q;
+        char *q = db <= V * sizeof(*s.z) ? (char *)s.z : (char *)s.r;
+        if (diffusion_own<T>(db, V, (size_t)nz * M)) NUDIM_TRY(s.alloc(&q, db));
+        if (db) s.diff = q;
     }
     s.part_stride = std::max(cgnr_part_stride(M, (int)P2), s.pl.toeplitz ? s.pl.nT / 4 : 0);
     NUDIM_TRY(s.alloc(&s.part, (size_t)nz * s.part_stride + 2 * (size_t)nz + 2));
@@ -696,9 +705,12 @@ static size_t job_bytes(const nudim_job_desc *d, int A, bool both, size_t fused_
         if (d->denoise == NUDIM_DENOISE_TV) b += V * sT;
         if (d->denoise == NUDIM_DENOISE_DIFFUSION) {
             const float lam = job_lambda(*d);
-            b += sT == 4 ? diffusion_scratch<float>(d->nz, d->np, d->np, lam, kJobKappa, kJobSweeps)
-                         : diffusion_scratch<double>(d->nz, d->np, d->np, lam, kJobKappa,
-                                                     kJobSweeps);
+            const size_t db = sT == 4 ? diffusion_scratch<float>(d->nz, d->np, d->np, lam, kJobKappa,
+                                                                 kJobSweeps)
+                                      : diffusion_scratch<double>(d->nz, d->np, d->np, lam, kJobKappa,
+                                                                  kJobSweeps);
+            if (sT == 4 ? diffusion_own<float>(db, V, nz * M) : diffusion_own<double>(db, V, nz * M))
+                b += db;
         }
         b += M * (8 + 28 * sT + 20);  // node tables and tile lists
         // fused-path lists: ~11 adjoint tile entries and <= 5 trafo entries per
