@@ -84,44 +84,41 @@ __device__ __forceinline__ float tv_inv(float z, float y, float x)
     return rsqrtf(__fmaf_rn(x, x, __fmaf_rn(y, y, __fmaf_rn(z, z, 1e-8f))));
 }
 
-// Quotients g / b of an update, b the gradient's norm.  FP32: from the rounded
-// reciprocal with two corrections, as the division rounds (the first brings the
-// quotient within one ulp, and from there one more correction with RN(1 / b)
-// rounds correctly: Markstein 1990; |g| is below 5, and values so small that a
-// residual underflows keep an error of an ulp).  FP64: intdiv.cuh.
+// An update's la (g / b), b the gradient's norm, rounded as the division and the
+// product round (intdiv.cuh; |g| is below 5).
 __device__ __noinline__ double tv_divided(double a, double b) { return rn_div(a, b); }
 
 template <typename T> struct TvNorm;
 template <> struct TvNorm<float> {
-    float b, y;
-    __device__ void init(float v)
+    float b, y, la;  // la: the factor, times 2^-64 where y is not 0
+    __device__ void init(float v, float l)
     {
         b = v;
-        y = v > 1e-15f && v < 1e15f ? __frcp_rn(v) : 0.f;
+        y = v > 1e-15f && v < 1e15f && l > 0x1p-60f ? __frcp_rn(v) : 0.f;
+        la = y == 0.f ? l : l * 0x1p-64f;
     }
-    __device__ __forceinline__ float quotient(float g) const
+    __device__ __forceinline__ float step(float g) const
     {
-        if (y == 0.f) return rn_div(g, b);  // the same for the whole launch
-        float q = rn_mul(g, y);
-        q = __fmaf_rn(__fmaf_rn(-q, b, g), y, q);
-        return __fmaf_rn(__fmaf_rn(-q, b, g), y, q);
+        if (y == 0.f) return rn_mul(la, rn_div(g, b));  // the same for the whole launch
+        return rn_mul(la, quotient64(g, b, y));
     }
 };
 template <> struct TvNorm<double> {
-    double b;
+    double b, la;
     IntDivisor d;
     bool ok;
-    __device__ void init(double v)
+    __device__ void init(double v, double l)
     {
         b = v;
+        la = l;
         ok = v > 1e-300 && v < 1e300;
         d = int_divisor(ok ? v : 1.0);
     }
-    __device__ __forceinline__ double quotient(double g) const
+    __device__ __forceinline__ double step(double g) const
     {
         double q;
         if (!(int_div(g, d, &q) && ok)) q = tv_divided(g, b);
-        return q;
+        return rn_mul(la, q);
     }
 };
 
@@ -249,7 +246,6 @@ k_tv_grad(const T *u, T *g, double *part,
         off[s] = (I)gj * nx + gk;
         upd[s] = c < kCells && (!height || (gj >= ylo && gj <= yhi));
     }
-    T la = T(0);
     T *const cells = &pl[0][0][0] + threadIdx.x, *const gcells = &plg[0][0] + threadIdx.x;
     // the planes of the run in order (the first and last clamped to the volume)
     // into ring slot `sl`; past the run's end only the group's count goes on
@@ -283,7 +279,7 @@ k_tv_grad(const T *u, T *g, double *part,
             for (int s = 0; s < kSlots; s++)
                 if (upd[s]) {
                     T *v = cells + sl * kCells + 256 * s;
-                    *v = rn_sub(*v, rn_mul(la, norm.quotient(gcells[sl * kCells + 256 * s])));
+                    *v = rn_sub(*v, norm.step(gcells[sl * kCells + 256 * s]));
                 }
         }
     };
@@ -295,8 +291,7 @@ k_tv_grad(const T *u, T *g, double *part,
     for (int q = 0; q < NS; q++) fetch(q);  // planes z0 - 1 .. z0 + NS - 2
     __pipeline_wait_prior(NS - 2);
     if (FUSED) {
-        norm.init((T)step_in[0]);
-        la = (T)step_in[1];
+        norm.init((T)step_in[0], (T)step_in[1]);
     }
     ready(0);
     ready(1);
@@ -478,8 +473,7 @@ k_tv_update(const T *u, T *u_out, const T *g, const double *step,
 {
     await_last();
     TvNorm<T> tn;
-    tn.init((T)step[0]);
-    const T la = (T)step[1];
+    tn.init((T)step[0], (T)step[1]);
     const I nv = (I)nz * ny * nx / VEC, stride = (I)gridDim.x * blockDim.x;
     for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < nv; t += stride) {
         TvVec<T, VEC> x = reinterpret_cast<const TvVec<T, VEC> *>(u)[t];
@@ -490,7 +484,7 @@ k_tv_update(const T *u, T *u_out, const T *g, const double *step,
                 int j = (int)(((t * VEC + e) / (I)nx) % (I)ny);
                 if (j < ylo || j > yhi) continue;
             }
-            x.v[e] = rn_sub(x.v[e], rn_mul(la, tn.quotient(y.v[e])));
+            x.v[e] = rn_sub(x.v[e], tn.step(y.v[e]));
         }
         reinterpret_cast<TvVec<T, VEC> *>(u_out)[t] = x;
     }

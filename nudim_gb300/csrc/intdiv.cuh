@@ -333,6 +333,26 @@ NUDIM_HD IntDivisor int_sqrt(double s)
     return d;
 }
 
+// ---------------------------------------------------------------- FP32 g / b
+// RN(2^64 g / b) from y = RN(1 / b), b in [1e-15, 1e15], |g| below 2^10: two
+// corrections (the first brings the quotient within one ulp, and from there one
+// more with RN(1 / b) rounds correctly: Markstein 1990).  The factor keeps the
+// residuals of the smallest g exact.
+NUDIM_HD float quotient64(float g, float b, float y)
+{
+#if defined(__CUDA_ARCH__)
+    const float h = __fmul_rn(g, 0x1p64f);
+    float q = __fmul_rn(h, y);
+    q = __fmaf_rn(__fmaf_rn(-q, b, h), y, q);
+    return __fmaf_rn(__fmaf_rn(-q, b, h), y, q);
+#else
+    const float h = g * 0x1p64f;
+    float q = h * y;
+    q = std::fma(std::fma(-q, b, h), y, q);
+    return std::fma(std::fma(-q, b, h), y, q);
+#endif
+}
+
 NUDIM_HD double double_of(const IntDivisor &d)
 {
     return double_of(((uint64_t)(uint32_t)(d.e + 1022) << 52) + d.n);
