@@ -233,10 +233,13 @@ def roofline_from_profile(prof, peak_gbs, peak_kind, r, csize, steps):
     - The Toeplitz CG's passes (k_toep_rows + k_toep_cols + k_toep_irows,
       class "toeplitz"): 11 per Z-plane and outer iteration (one before the
       loop, one per step).  Unit: one Z-plane's operator pass, c (3 P^2 +
-      4 P nt) bytes -- p in, T p out and p read again for p^H T p, and the
-      P x nt row spectra written, read and written by the column pass, and
-      read back (nt: the circulant's size, 768 for P = 384).  The vector
-      updates that ride on the row passes (another 4 P^2) are not counted.
+      4 P nt) bytes -- p in, z in and z - alpha T p out, and the P x nt row
+      spectra written, read and written by the column pass, and read back
+      (nt: the circulant's size, 768 for P = 384).  The vector updates that
+      ride on the forward row pass are left out of the unit; with_updates has
+      them too: z in, p out, f in and out in the steps after the first
+      (7 P^2 in all), 4 P^2 in the first (p = z), 3.5 P^2 in the pass before
+      the loop (a real start value in, f out, z in and out).
     - The adjoint NFFT (k_spread_gather + k_spread_fixup + k_colifft_fs +
       k_rowifft_crop_fs, classes "spread" + "crop"): 11 per Z-plane and outer
       iteration with the NFFT form of the CGNR, 1 with the Toeplitz form.
@@ -257,21 +260,27 @@ def roofline_from_profile(prof, peak_gbs, peak_kind, r, csize, steps):
         nt = 768 if (2 * P - 1 <= 768 < n and os.environ.get("NUDIM_TOEPLITZ_GRID") != "nfft") else n
         unit = csize * (3 * P * P + 4 * P * nt)
         tr = MEASURED_TOEPLITZ_TRAFFIC_PER_PLANE.get(nt)
+        full = csize * ((3.5 + 4 + 7 * 9) / 11 * P * P + 4 * P * nt)
         groups.append(("Toeplitz operator pass",
                        "Toeplitz CG step (k_toep_rows + k_toep_cols + k_toep_irows)",
-                       toep[0], units, launches, unit, tr))
+                       toep[0], units, launches, unit, tr, full))
     ms_s, n_s, _ = prof["spread"]
     ms_c, n_c, _ = prof["crop"]
     units = (1 if toep[1] > 0 else 11) * nz * steps
     groups.append(("adjoint NFFT",
                    "adjoint NFFT (k_spread_gather + k_spread_fixup + k_colifft_fs + "
                    "k_rowifft_crop_fs)", ms_s + ms_c, units, max(1, n_c),
-                   csize * (P * P + 4 * n * n + M), MEASURED_ADJOINT_TRAFFIC_PER_PLANE))
-    top, kernel, ms, units, launches, unit, tr = max(groups, key=lambda g: g[2])
+                   csize * (P * P + 4 * n * n + M), MEASURED_ADJOINT_TRAFFIC_PER_PLANE, None))
+    top, kernel, ms, units, launches, unit, tr, full = max(groups, key=lambda g: g[2])
     planes_per_launch = units / launches
     achieved = units * unit / (ms / 1e3) / 1e9
+    updates = {}
+    if full:
+        rate = units * full / (ms / 1e3) / 1e9
+        updates["with_updates"] = {"bytes_per_unit": round(full), "achieved": round(rate, 1),
+                                   "frac": round(rate / peak_gbs, 4)}
     return top, {
-        "bound": "hbm", "kernel": kernel,
+        "bound": "hbm", "kernel": kernel, **updates,
         "achieved": round(achieved, 1), "peak": peak_gbs, "unit": "GB/s",
         "frac": round(achieved / peak_gbs, 4),
         "traffic": round(tr * planes_per_launch) if tr else None,
