@@ -463,9 +463,8 @@ template <typename T, int N> struct alignas(sizeof(T) * N) TvVec {
 };
 
 // u_out = u - (lam * sqrt(dA)) * (g / sqrt(sum g^2))   (denoise.c:125-142),
-// VEC voxels per access; u_out may be u.  The two scalars are formed once per
-// block (the same FP64 expressions in every block, so every voxel sees the
-// same values).
+// VEC voxels per access; u_out may be u.  step: the norm and the factor, as the
+// gradient pass left them.
 template <typename T, typename I, int VEC>
 __global__ void __launch_bounds__(256)
 k_tv_update(const T *u, T *u_out, const T *g, const double *step,

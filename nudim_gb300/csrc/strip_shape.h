@@ -19,23 +19,24 @@ template <typename T> constexpr int kBandRows = sizeof(T) == 4 ? 384 : 64;
 // The next launch's shape with `left` sweeps to go.
 //
 // FP32: 16 live sweeps (or what 16 warps hold): more of them waste more on the
-// pipeline's ends, fewer leave the SM idle (256 x 384 x 384: 8 sweeps 4.29, 10
-// 5.09, 16 4.15, 20 5.51 ms).  Two sweeps a warp halve the exchange and let two
+// pipeline's ends, fewer leave the SM idle (256 x 384 x 384: 8 sweeps 4.60, 10
+// 5.28, 16 4.40, 20 5.84 ms).  Two sweeps a warp halve the exchange and let two
 // CTAs share an SM; with a plane per SM or fewer, one sweep a warp on twice the
-// warps (64 x 128 x 128: 386 -> 363 us; 256 planes of 384 x 384: 4.15 -> 4.93
-// ms the other way round).  Where four CTAs a plane still find an SM each and
-// the strips are at least 6 rows, a cluster of four with 40 live sweeps (33 x
-// 151 x 203: 753 -> 586 us; 16 x 64 x 64, strips of 2 rows: 154 -> 206 us, the
-// cluster's barrier at each step costs more than the rest of the step).
+// warps (64 x 128 x 128: 386 -> 335 us, 96 x 384 x 384 2.65 -> 2.28 ms; 256
+// planes of 384 x 384: 4.40 -> 4.56 ms the other way round).  Where four CTAs a
+// plane still find an SM each and the strips are at least 6 rows, a cluster of
+// four with 40 live sweeps (33 x 151 x 203: 715 -> 592 us; 16 x 64 x 64, strips
+// of 2 rows: 145 -> 208 us, the cluster's barrier at each step costs more than
+// the rest of the step).
 //
 // FP64: the step is long (integer and FP64 units; 64 x 128 x 128: 38.0 ms for
 // the tables form with the FP64 unit's divisions, 4.0 here) and a plane on one
 // SM leaves the others idle, so a plane takes a cluster of as many CTAs as
-// bring the turns per SM down (64 planes: 1 CTA 7.3 ms, 2 4.05, 4 3.96, 8 3.98;
-// 32: 4 2.64, 8 2.54; equal turns: the smaller one), strips of 2 rows on up to
+// bring the turns per SM down (64 planes: 1 CTA 7.32 ms, 2 3.97, 4 3.94, 8 3.96;
+// 32: 4 2.63, 8 2.55; equal turns: the smaller one), strips of 2 rows on up to
 // 16 warps (strips of 4 on half the warps: 6.6 against 5.3 ms, one warp's
 // dependent instructions bound it), 16 live sweeps; 40 where there are fewer
-// planes than clusters of 8 (9 x 100 x 130: 1.93 -> 1.71 ms).
+// planes than clusters of 8 (9 x 100 x 130: 1.93 -> 1.70 ms).
 template <typename T> StripShape strip_shape(int nz, int ny, int nx, int left, int sms)
 {
     StripShape s;

@@ -26,11 +26,16 @@
 // Bound: issue and the FMA, ALU and special-function pipes together (25
 // instructions a cell, of 38 cycles a warp's 32 cells take on a scheduler; the
 // boundary columns' selects are a quarter of them).  256 x 384 x 384, 80
-// sweeps: 4.15 ms against 12.1 ms for the shared-memory pairs form.
+// sweeps: 4.40 ms against 12.1 ms for the shared-memory pairs form.
 // The cell's four coefficients K^2 / (K^2 + g^2) are summed in pairs over a
 // common denominator, gN/dN + gS/dS = (gN dS + gS dN) / (dN dS): one reciprocal
 // for two coefficients (four per cell bound the loop by the special-function
-// unit at 4 cells per clock and SM).  FP64 by the integer units (66 % of their
+// unit at 4 cells per clock and SM: 5.30 ms).  The distance from FP64 results,
+// against that of the pairs form with its reciprocal per neighbour: median 0.99,
+// geometric mean 1.00 times it over 150 volumes of 9 thousand to 11 million voxels
+// (ragged, planes of 32 to 384 a side; lambda 1/4), 1.02 on 256 x 384 x 384, 0.7 where lambda
+// is 0.4; one reciprocal refined by a step of Newton's iteration 1.01 there, at
+// 4.61 ms.  FP64 by the integer units (66 % of their
 // rate) and the FP64 unit (67 %), see intdiv.cuh.
 #include <cooperative_groups.h>
 
@@ -81,8 +86,7 @@ template <> struct CellArgs<double> {
 
 // Cells of two adjacent rows.  The differences are scalar:
 // the rows' N and S are not a register pair, and pairing rows (i, i + R/2),
-// whose N and S are, took more moves than it saved (256 x 384 x 384: 4.15 ->
-// 4.47 ms).
+// whose N and S are, took more moves than it saved (256 x 384 x 384: 8 % slower).
 __device__ __forceinline__ void cell2(float c0, float c1, float n0, float n1, float s0, float s1,
                                       float e0, float e1, float w0, float w1,
                                       const CellArgs<float> &k, float &u0, float &u1)
