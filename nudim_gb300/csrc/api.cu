@@ -310,7 +310,7 @@ template <typename T> static int state_init(nudim_job *jb, JobState<T> &s)
         if (diffusion_own<T>(db, V, (size_t)nz * M)) NUDIM_TRY(s.alloc(&q, db));
         if (db) s.diff = q;
     }
-    s.part_stride = std::max(cgnr_part_stride(M, (int)P2), s.pl.toeplitz ? s.pl.nT / 4 : 0);
+    s.part_stride = std::max(s.pl.part_stride(), s.pl.toeplitz ? s.pl.nT / 4 : 0);
     NUDIM_TRY(s.alloc(&s.part, (size_t)nz * s.part_stride + 2 * (size_t)nz + 2));
     NUDIM_TRY(s.alloc(&s.dots, (size_t)nz * 4));
     NUDIM_TRY(s.alloc(&s.rh, (size_t)std::max(1, jb->d.nhio + jb->d.ner)));
@@ -1473,7 +1473,7 @@ static int op_cgnr(nudim_nfft_plan *p, NfftDev<T> &d, int nplanes, const void *y
 {
     using C = cplx_t<T>;
     size_t N = (size_t)d.N0 * d.N1, M = d.M;
-    int stride = cgnr_part_stride((int)M, (int)N);
+    const int stride = d.part_stride();
     size_t need = sizeof(C) * nplanes * (2 * M + 2 * N) +
                   sizeof(double) * ((size_t)nplanes * (stride + 4) + 8);
     if (need > p->cg_bytes) {

@@ -11,6 +11,7 @@
 //   grid workspace chunk*n0*n1 complex, owned by the context
 #pragma once
 
+#include <algorithm>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -218,6 +219,9 @@ template <typename T> struct NfftDev {
     {
         return fused ? ceil_div(N0, rows) : ceil_div((long)N0 * N1, 256);
     }
+    // a plane's partial sums at most: two per block of nodes, one per block of
+    // coefficients (few nodes on many rows: more of these)
+    int part_stride() const { return std::max(2 * interp_blocks(), crop_blocks()); }
     int trafo(int nplanes, const PadArgs<T> &pa, const InterpArgs<T> &ia, cudaStream_t st);
     int adjoint(int nplanes, const SpreadArgs<T> &sa, const CropArgs<T> &ca, cudaStream_t st);
 
