@@ -184,6 +184,12 @@ int build_nfft_tables(int N0, int N1, int M, const double *x, int ty, int tx, Nf
                     for (int s = 0; s < kW; s++) ps[s] = q[s];
                 } else {
                     for (int s = 0; s < kW; s++) ps[s] = kb_phi(xn - (double)(u + s), b);
+                    // a grid shorter than the window: taps that meet the same
+                    // point as one (the adjoint's lists look a point's weight up)
+                    for (int s = n; s < kW; s++) {
+                        ps[s % n] += ps[s];
+                        ps[s] = 0.0;
+                    }
                 }
             }
         }
