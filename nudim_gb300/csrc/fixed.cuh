@@ -57,6 +57,13 @@ NUDIM_HD Fixed fixed_shift(Fixed a, int s)
     return split_fixed((V + ((1ll << s) >> 1)) >> s);
 }
 
+// 2^s a, s <= 2, exactly: not split anew (the parts grow; 14 products of such
+// weights still fit FixedSum's 64 bits)
+NUDIM_HD Fixed fixed_scaled(Fixed a, int s)
+{
+    return Fixed{(int)((uint32_t)a.hi << s), (int)((uint32_t)a.lo << s)};
+}
+
 // the product of two numbers under exponent field E, under field 2 E - 1022
 NUDIM_HD Fixed fixed_product(Fixed a, Fixed b)
 {

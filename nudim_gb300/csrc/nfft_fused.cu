@@ -184,8 +184,9 @@ __device__ __forceinline__ bool fix_columns(double2 *G, int stride, int n, int B
 // A node's window over the block's columns in the FP64 form: row weights as
 // fixed point (exponent field Ew), column q of the entry at gp(q). The rows are
 // summed in integers, the columns in FP64 (those in integers too: as long, and an
-// error up to twice as large). The window's 14 rows lie in at most two groups: the
-// weights of the one with the smaller values are shifted to the other's field.
+// error up to twice as large). The window's 14 rows lie in at most two groups.
+// Bounds up to 4 times apart: the larger one's weights are scaled up, exactly;
+// further apart: the smaller one's are shifted to the other's field.
 template <typename F>
 __device__ __forceinline__ double2 window_fp64(const double *__restrict__ qa,
                                                const double *__restrict__ q1, size_t nE, int e,
@@ -201,10 +202,13 @@ __device__ __forceinline__ double2 window_fp64(const double *__restrict__ qa,
         for (int i = 0; i < 14; i++) w[i] = *reinterpret_cast<const Fixed *>(qa + i * nE);
         const int r0 = (rb + odd) & m0, here = kFixRows - r0 % kFixRows;  // rows of the first group
         const int Ea = she[r0 / kFixRows], Eb = she[((r0 + 13) & m0) / kFixRows];
-        const int E = max(Ea, Eb);
-        if (Ea != Eb) {
+        const int lo = min(Ea, Eb), hi = max(Ea, Eb), E = hi - lo <= 2 ? lo : hi;
+        if (hi - lo > 2) {
 #pragma unroll
-            for (int i = 0; i < 14; i++) w[i] = fixed_shift(w[i], E - (i < here ? Ea : Eb));
+            for (int i = 0; i < 14; i++) w[i] = fixed_shift(w[i], hi - (i < here ? Ea : Eb));
+        } else if (hi != lo) {
+#pragma unroll
+            for (int i = 0; i < 14; i++) w[i] = fixed_scaled(w[i], (i < here ? Ea : Eb) - lo);
         }
         for (int q = 0; q < cnt; q++) {
             const FixedC *g = reinterpret_cast<const FixedC *>(gp(q));

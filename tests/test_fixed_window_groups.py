@@ -28,6 +28,17 @@ extern "C" double window(const double *w, const double *v, int n, int here, int 
     }
     return s.re() * fixed_scale(Ew, E);
 }
+extern "C" double window_near(const double *w, const double *v, int n, int here, int Ew, int Ea, int Eb)
+{
+    FixedSum s;
+    s.init();
+    const int E = Ea < Eb ? Ea : Eb;
+    for (int i = 0; i < n; i++) {
+        const int Ei = i < here ? Ea : Eb;
+        s.add(fixed_scaled(to_fixed(w[i], Ew), Ei - E), FixedC{to_fixed(v[i], Ei), Fixed{0, 0}});
+    }
+    return s.re() * fixed_scale(Ew, E);
+}
 extern "C" int shifted(int hi, int lo, int s, int *olo)
 {
     const Fixed f = fixed_shift(Fixed{hi, lo}, s);
@@ -48,7 +59,8 @@ def host(tmp_path_factory):
                     so], check=True)
     lib = ctypes.CDLL(so)
     p, i = ctypes.c_void_p, ctypes.c_int
-    lib.window.restype, lib.window.argtypes = ctypes.c_double, [p, p, i, i, i, i, i]
+    for fn in (lib.window, lib.window_near):
+        fn.restype, fn.argtypes = ctypes.c_double, [p, p, i, i, i, i, i]
     lib.shifted.restype, lib.shifted.argtypes = i, [i, i, i, p]
     return lib
 
@@ -85,6 +97,30 @@ def test_window_of_two_groups_against_exact(host, gap, here, first):
         exact = sum(Fraction(x) * Fraction(y) for x, y in zip(w, v))
         bound = Fraction(2) ** (Ew - 1022 + max(Ea, Eb) - 1022)
         assert abs(Fraction(got) - exact) <= 14 * bound / 2 ** 55 + abs(exact) / 2 ** 53
+
+
+@pytest.mark.parametrize("gap", [0, 1, 2])
+@pytest.mark.parametrize("here", [1, 7, 13])
+@pytest.mark.parametrize("extreme", [0, 1])
+def test_window_of_near_bounds_against_exact(host, gap, here, extreme):
+    """Bounds up to 4 times apart, the larger one's weights scaled exactly: the same
+    error without the shift's part, and no overflow where every operand is the
+    largest of its field."""
+    rng = np.random.default_rng(gap + 10 * here)
+    for first in (0, 1):
+        for _ in range(20):
+            w, v = rng.random(14) * 3e9, rng.standard_normal(14)
+            if extreme:
+                w = np.full(14, np.nextafter(2.0 ** 33, 0)) * rng.choice([-1, 1])
+                v = np.full(14, np.nextafter(1.0, 0)) * rng.choice([-1, 1])
+            v[(np.arange(14) < here) == bool(first)] *= 2.0 ** -gap
+            Ea, Eb, Ew = field(v[:here]), field(v[here:]), field(w)
+            if abs(Ea - Eb) > 2:
+                continue
+            got = host.window_near(w.ctypes.data, v.ctypes.data, 14, here, Ew, Ea, Eb)
+            exact = sum(Fraction(x) * Fraction(y) for x, y in zip(w, v))
+            bound = Fraction(2) ** (Ew - 1022 + max(Ea, Eb) - 1022)
+            assert abs(Fraction(got) - exact) <= 14 * bound / 2 ** 55 + abs(exact) / 2 ** 53
 
 
 def both(ctx, ng, monkeypatch, n, x, fh, y):
