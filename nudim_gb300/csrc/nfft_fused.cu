@@ -404,7 +404,7 @@ k_colfft_interp(const cplx_t<T> *H, int N0, int n0, int logn0, int n1, int BC,
 // banks); then every thread interpolates as in k_colfft_interp. FP64 (the FP32
 // form has the kernels below). The FP64 unit's FFTs and the integer sums of
 // other CTAs overlap: two CTAs an SM where the registers allow (n0 = 256; 24
-// planes at 128^2: 344 -> 235 us, 259 with a bound per group of rows).
+// planes at 128^2: 344 -> 235 us, 256 with a bound per group of rows).
 template <int R1, int R2>
 __global__ void __launch_bounds__(32 * col_warps<double>(), R1 == 16 ? 2 : 1)
 k_colfft_interp_fs(const double2 *H, int N0, int n1,
